@@ -6,8 +6,8 @@
 // queue (one atomic counter) and, for every block of its tile, marches the
 // block's rays 32 at a time (one lane per ray, the count-down march with
 // Kahan columns) and integrates their rates at once (exact FP32 quadrature,
-// eight lanes per ray), so the columns never leave the registers; lane j
-// sums the rays of cell j of the block in ray order.  The arithmetic is
+// the warp on one ray after another), so the columns never leave the SM; lane
+// j sums the rays of cell j of the block in ray order.  The arithmetic is
 // that of argot_b200_march_rays + argot_b200_photoion_rays (EXACT_F32), so
 // every problem's rates equal those of the problem run alone, bit for bit.
 //
@@ -57,26 +57,19 @@ struct BatchItem {
 
 // Launch shape: kWarps warps per CTA and at least ARGOT_BATCH_MIN_WARPS / kWarps
 // CTAs resident per SM (which caps the registers per thread).  Measured on
-// B200 (the 48-problem batch): 32 warps per SM (64 registers) run the step
-// 22% faster than 16.
+// B200 (8 problems of 32^3 to 96^3 cells): 24 warps per SM (80 registers)
+// 78.4 ms, 16 warps 81.0 ms, 32 warps (64 registers, spilling the rates'
+// tables) 89.5 ms.
 #ifndef ARGOT_BATCH_MIN_WARPS
-#define ARGOT_BATCH_MIN_WARPS 32
+#define ARGOT_BATCH_MIN_WARPS 24
 #endif
 template <int kWarps>
 __global__ void __launch_bounds__(32 * kWarps, ARGOT_BATCH_MIN_WARPS / kWarps)
     k_batch(const BatchProb *__restrict__ probs, const BatchItem *__restrict__ items, uint32_t nitems,
             uint32_t *__restrict__ next, unsigned long long *__restrict__ crossings, int *__restrict__ err) {
-  __shared__ BinPair s_pairs[kBinPairs];
-  __shared__ float s_nd[kWarps][32][6];
-  __shared__ float s_p[kWarps][32][3];
-  __shared__ float s_out[kWarps][32][6];
-  __shared__ int s_e[kWarps][32], s_t[kWarps][32], s_cnt[kWarps][32], s_src[kWarps][32];
-  __shared__ int s_nsfu[kWarps][32];
-  load_bin_pairs(s_pairs);
-  __syncthreads();
+  __shared__ RateChunk s_c[kWarps];
+  __shared__ int s_cnt[kWarps][32], s_src[kWarps][32];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int grp = lane >> 3, j = lane & 7;
-  const unsigned gmask = 0xffu << (8 * grp);
   unsigned long long steps_total = 0;
   bool bad = false;
   for (;;) {
@@ -126,44 +119,20 @@ __global__ void __launch_bounds__(32 * kWarps, ARGOT_BATCH_MIN_WARPS / kWarps)
           const float4 rw = __ldg(raw + cell_index(g, lx, ly, lz));
           const RayParams p = ray_params_f32(g, g.ix0 + lx, g.iy0 + ly, g.iz0 + lz, ep.x, ep.y, ep.z, tt.hi, tt.hei,
                                              tt.heii, rw, __ldg(total + e));
+          s_c[wib].rec[lane] = ray_rec(p, (int)e);
 #pragma unroll
-          for (int s = 0; s < 3; s++) {
-            s_nd[wib][lane][s] = p.N[s];
-            s_nd[wib][lane][3 + s] = p.D[s];
-            s_p[wib][lane][s] = p.P[s];
-          }
-          s_e[wib][lane] = (int)e;
-          s_nsfu[wib][lane] = sfu_iters(p.D[0], p.D[1], p.D[2]);
-        }
-        s_t[wib][lane] = t;
-        __syncwarp();
-        const int nk = (int)min((uint64_t)32, r1 - rc);
-        // rounds of four rays with one SFU count, as in rate_block_f32
-        for (int q0 = 0; q0 < nk; q0 += 4) {
-          const int q = q0 + grp < nk ? q0 + grp : q0;
-          int nsfu = 0;
-#pragma unroll
-          for (int k = 0; k < 4; k++) nsfu = max(nsfu, q0 + k < nk ? s_nsfu[wib][q0 + k] : 0);
-          const float N0 = s_nd[wib][q][0], N1 = s_nd[wib][q][1], N2 = s_nd[wib][q][2];
-          const float D0 = s_nd[wib][q][3], D1 = s_nd[wib][q][4], D2 = s_nd[wib][q][5];
-          const float *sp = specn + (size_t)s_e[wib][q] * kNu;
-          float part[6];
-          ray_bins_packed(s_pairs, sp, j, nsfu, s_nsfu[wib][q], N0, N1, N2, D0, D1, D2, part);
-#pragma unroll
-          for (int o = 1; o < 8; o <<= 1) {
-#pragma unroll
-            for (int s = 0; s < 6; s++) part[s] += __shfl_xor_sync(gmask, part[s], o);
-          }
-          if (j == 0 && q0 + grp < nk) {
-            const float Pq[3] = {s_p[wib][q][0], s_p[wib][q][1], s_p[wib][q][2]};
-            float out[6];
-            ray_rates6(Pq, part[0], part[1], part[2], part[3], part[4], part[5], out);
-#pragma unroll
-            for (int s = 0; s < 6; s++) s_out[wib][q][s] = out[s];
-          }
+          for (int s = 0; s < 3; s++) s_c[wib].p[lane][s] = p.P[s];
         }
         __syncwarp();
-        add_chunk_in_order(acc, lane, t, s_out[wib], s_cnt[wib], s_src[wib]);
+        {
+          // the lane's cross sections, read again for every chunk so that
+          // the march does not carry them
+          RateLane tab;
+          load_rate_lane(lane, tab);
+          chunk_rates(s_c[wib], tab, specn, nullptr, (int)min((uint64_t)32, r1 - rc), lane);
+        }
+        __syncwarp();
+        add_chunk_in_order(acc, lane, t, s_c[wib].out, s_cnt[wib], s_src[wib]);
       }
       if (own_valid) {
 #pragma unroll
@@ -188,12 +157,9 @@ __global__ void __launch_bounds__(32 * kWarps, ARGOT_BATCH_MIN_WARPS / kWarps)
 #define ARGOT_SPLIT_MARCH_MIN_CTAS 6
 #endif
 #ifndef ARGOT_SPLIT_RATE_MIN_CTAS
-#define ARGOT_SPLIT_RATE_MIN_CTAS 2
+#define ARGOT_SPLIT_RATE_MIN_CTAS 4
 #endif
-#ifndef ARGOT_SPLIT_RATE_RAYS_PER_LANE
-#define ARGOT_SPLIT_RATE_RAYS_PER_LANE 2
-#endif
-constexpr int kSplitRateWarps = 8;
+constexpr int kSplitRateWarps = 4;
 
 __global__ void __launch_bounds__(256, ARGOT_SPLIT_MARCH_MIN_CTAS)
     k_batch_march(const BatchProb *__restrict__ probs, const BatchItem *__restrict__ items, uint32_t i0,
@@ -242,11 +208,10 @@ __global__ void __launch_bounds__(256, ARGOT_SPLIT_MARCH_MIN_CTAS)
 __global__ void __launch_bounds__(32 * kSplitRateWarps, ARGOT_SPLIT_RATE_MIN_CTAS)
     k_batch_rates(const BatchProb *__restrict__ probs, const BatchItem *__restrict__ items, uint32_t i0,
                   uint32_t i1, uint32_t *__restrict__ next) {
-  __shared__ BinPair s_pairs[kBinPairs];
   __shared__ RateWarpSmem s_w[kSplitRateWarps];
-  load_bin_pairs(s_pairs);
-  __syncthreads();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  RateLane tab;
+  load_rate_lane(lane, tab);
   for (;;) {
     uint32_t it = 0;
     if (lane == 0) it = i0 + atomicAdd(next, 1u);
@@ -256,9 +221,8 @@ __global__ void __launch_bounds__(32 * kSplitRateWarps, ARGOT_SPLIT_RATE_MIN_CTA
     const BatchProb &P = probs[wi.prob];
     const GridDev g = P.g;
     for (uint64_t b = wi.b0; b < wi.b1; b++)
-      rate_block_f32<false, ARGOT_SPLIT_RATE_RAYS_PER_LANE>(g, P.raw, P.emit_pos, P.specn, P.total, s_pairs, b,
-                                                            P.blk_off[b], P.blk_off[b + 1], P.rays, P.nray, P.tau,
-                                                            P.rates6, s_w[wib], lane);
+      rate_block_f32<false>(g, P.raw, P.emit_pos, P.specn, P.total, tab, b, P.blk_off[b], P.blk_off[b + 1], P.rays,
+                            P.nray, P.tau, P.rates6, s_w[wib], lane);
   }
 }
 

@@ -56,10 +56,9 @@ struct RateTables {
   float cs[3][kNu];       // sigma_s(nu) [cm^2]
   float cs_l2e[3][kNu];   // sigma_s(nu) * log2(e)
   float hw[3][kNu];       // sigma_s(nu) * max((float)nu - nu_s, 0)
-  float smax16[3][16];    // max of sigma_s(nu) over the bins k >= 16 i
-  // the bin loop's iterations (16 bins each) before iter_he have sigma_HeI =
-  // sigma_HeII = 0 in every bin, those before iter_heii sigma_HeII = 0
-  int iter_he, iter_heii;
+  float hw_l2e[3][kNu];   // sigma_s(nu) * log2(e) * max((float)nu - nu_s, 0)
+  // max of sigma_s(nu) over the bins k >= 64 m (the stages of the FP32 loop)
+  float smax[3][4];
 };
 // Uploads the tables to the constant bank of the translation unit that owns
 // the rate kernels (photoion.cu), once per device.
@@ -77,12 +76,11 @@ void host_tables(double *nu, float *cs3);
 // sigma_s(nu) * ((float)nu - nu_s)^+ for s = HI, HeI, HeII.
 void host_rate_weights(double *w6);
 
-// Position of bin k in an emitter's normalised spectrum (emit_specn): the
-// bins are stored in the pair order of the packed rate loop, pair
-// p = (k % 8) + 8 (k / 16) holding bins k0 = (p % 8) + 16 (p / 8) and k0 + 8
-// at 2 p and 2 p + 1, so one 8-byte load fetches a pair.
-__host__ __device__ __forceinline__ int spec_pair_index(int k) {
-  return 2 * ((k & 7) + 8 * (k >> 4)) + ((k >> 3) & 1);
+// Position of bin k in an emitter's normalised spectrum (emit_specn): lane l
+// of a warp integrates the bins 64 m + l and 64 m + l + 32, m = 0..3, and
+// finds them at 8 l + 2 m and 8 l + 2 m + 1, 32 bytes it reads at once.
+__host__ __device__ __forceinline__ int spec_lane_index(int k) {
+  return 8 * (k & 31) + 2 * (k >> 6) + ((k >> 5) & 1);
 }
 
 // Emitters and tree on the device.
@@ -106,7 +104,7 @@ struct argot_b200_dev_tree {
   float4 *emit_pos;        // n_emit (x, y, z, 0)
   float emit_lo[3], emit_hi[3];  // bounding box of the emitter positions
   double *emit_spec64;     // n_emit x 256
-  float *emit_specn;       // n_emit x 256: spectrum / total, in bin-pair order (spec_pair_index)
+  float *emit_specn;       // n_emit x 256: spectrum / total, in lane order (spec_lane_index)
   double *emit_total;      // n_emit
   // surrogate inputs (set by argot_b200_dev_tree_set_blackbody): log10 T of
   // an emitter whose spectrum is a single-temperature blackbody (NaN

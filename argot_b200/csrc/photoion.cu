@@ -80,38 +80,18 @@ __global__ void __launch_bounds__(32 * kRateWarps)
 }
 
 // ------------------------------------------------------------ FP32 rates
-// One warp per target block, rays in chunks of 32.  Phase A: lane i forms
-// the FP32 per-ray parameters of ray i of the chunk (ray_params_f32).
-// Phase B: the warp splits into four groups of eight lanes; a group takes
-// ARGOT_RATE_RAYS_PER_LANE rays at a time and its lanes share the 256
-// frequency bins (lane j: bins j, j+8, ..., two at a time with the packed
-// f32x2 arithmetic, ray_bins_packed2), reading the bin-pair table from
-// shared memory; three butterfly steps sum the eight partial sums.  Phase C: every lane adds the
-// rays that end in its cell, in ray order (add_chunk_in_order).  The
+// One warp per target block, rays in chunks of 32 (rate_block_f32).  The
 // kernel has no FP64 arithmetic.
 // Launch shape: ARGOT_RATE_WARPS warps per CTA, at least ARGOT_RATE_MIN_CTAS
-// CTAs resident per SM (which caps the registers per thread), and
-// ARGOT_RATE_RAYS_PER_LANE rays per 8-lane group in phase B.  Measured on
-// B200 (256^3, 4096 sources, 3.2e9 rays) with the per-cell sums in shared
-// memory: one ray per group, 8 warps x 3 CTAs (80 registers, no spills)
-// 0.93 s; two rays per group, 8 warps x 2 CTAs (112 registers) 0.85 s,
-// x 3 CTAs (80 registers, spilling) 0.94 s.  With the later bin loop (the
-// mid-cell form, the 48-byte table, the species stretches, 4-fold unroll)
-// two rays per group at 8 warps x 2 CTAs (126 registers) take 0.75 s, at
-// 4 warps x 4 CTAs 0.78 s; but the smaller CTAs share the SMs better with
-// the march in the overlapped step, which runs 1.2% faster with them
-// (1.437 s against 1.454 s); 4 warps x 5 CTAs (96 registers, the
-// polynomial iterations unrolled twice, no spills) run the rates alone in
-// the same time and the step 2.3% faster again (1.403 s; unrolled four
-// times at 5 CTAs the loop spills: rates 0.83 s, step 1.435 s).
+// CTAs resident per SM (which caps the registers per thread).  Measured on
+// B200 (256^3 cells, 1024 sources): 4 warps x 4 CTAs (124 registers, no
+// spills) 0.471 s, the step with the march 0.977 s; x 5 CTAs (96 registers)
+// 0.524 s and 1.011 s.
 #ifndef ARGOT_RATE_WARPS
 #define ARGOT_RATE_WARPS 4
 #endif
 #ifndef ARGOT_RATE_MIN_CTAS
-#define ARGOT_RATE_MIN_CTAS 5
-#endif
-#ifndef ARGOT_RATE_RAYS_PER_LANE
-#define ARGOT_RATE_RAYS_PER_LANE 2
+#define ARGOT_RATE_MIN_CTAS 4
 #endif
 constexpr int kF32Warps = ARGOT_RATE_WARPS;
 
@@ -122,11 +102,10 @@ __global__ void __launch_bounds__(32 * kF32Warps, ARGOT_RATE_MIN_CTAS)
                const uint64_t *__restrict__ blk_off, uint64_t base, const uint32_t *__restrict__ rays,
                uint64_t nray, const float *__restrict__ tau, float *__restrict__ rates6,
                const float *__restrict__ pred, int *__restrict__ err) {
-  __shared__ BinPair s_pairs[kBinPairs];
   __shared__ RateWarpSmem s_w[kF32Warps];
-  load_bin_pairs(s_pairs);
-  __syncthreads();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  RateLane tab;
+  load_rate_lane(lane, tab);
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarp = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   for (uint64_t b = b0 + warp; b < b1; b += nwarp) {
@@ -135,8 +114,8 @@ __global__ void __launch_bounds__(32 * kF32Warps, ARGOT_RATE_MIN_CTAS)
       if (lane == 0) atomicExch(err, 1);
       continue;
     }
-    rate_block_f32<kServed, ARGOT_RATE_RAYS_PER_LANE>(g, raw, emit_pos, specn, total, s_pairs, b, r0, r1, rays,
-                                                      nray, tau, rates6, s_w[wib], lane, pred);
+    rate_block_f32<kServed>(g, raw, emit_pos, specn, total, tab, b, r0, r1, rays, nray, tau, rates6, s_w[wib], lane,
+                            pred);
   }
 }
 

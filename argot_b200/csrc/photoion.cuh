@@ -15,6 +15,15 @@ constexpr double kHNuL = kHPlanck * kNuL;  // hplanck*nuL, double
 // own ensure_rate_tables().
 __constant__ RateTables c_tab;
 
+// The FP32 bin loop's table: of stage m (bins 64 m .. 64 m + 63) the two bins
+// 64 m + l and 64 m + l + 32 of lane l; value s: sigma_s log2(e), value
+// 3 + s: sigma_s log2(e) (nu - nu_s)^+.
+constexpr int kStages = 4;
+struct RateTab {
+  float2 v[kStages][6][32];
+};
+static __device__ RateTab d_rate_tab;
+
 static int ensure_rate_tables(int device) {
   static std::mutex mu;
   static bool done[64] = {false};
@@ -36,24 +45,26 @@ static int ensure_rate_tables(int device) {
       t.cs_l2e[s][i] = (float)((double)c * l2e);
       const double w = ((double)nf > thr[s]) ? ((double)nf - thr[s]) : 0.0;
       t.hw[s][i] = (float)((double)c * w);
+      t.hw_l2e[s][i] = (float)((double)c * l2e * w);
     }
   }
-  // suffix maxima of the cross sections per 16-bin iteration (sfu_iters)
-  // and the iterations below the helium thresholds (sigma_s is 0 below
-  // nu_s in the fits of prim_chem/cross_section.c)
-  int first[3];
   for (int s = 0; s < 3; s++) {
     float m = 0.f;
-    first[s] = kNu / 16;
     for (int k = kNu - 1; k >= 0; k--) {
       m = fmaxf(m, t.cs[s][k]);
-      if (k % 16 == 0) t.smax16[s][k / 16] = m;
-      if (t.cs[s][k] != 0.f) first[s] = k / 16;
+      if (k % 64 == 0) t.smax[s][k / 64] = m;
     }
   }
-  t.iter_heii = first[2];
-  t.iter_he = std::min(first[1], first[2]);
   ARGOT_CUDA_TRY(cudaMemcpyToSymbol(c_tab, &t, sizeof(t)));
+  RateTab rt;
+  for (int m = 0; m < kStages; m++)
+    for (int l = 0; l < 32; l++)
+      for (int s = 0; s < 3; s++) {
+        const int k0 = 64 * m + l, k1 = k0 + 32;
+        rt.v[m][s][l] = make_float2(t.cs_l2e[s][k0], t.cs_l2e[s][k1]);
+        rt.v[m][3 + s][l] = make_float2(t.hw_l2e[s][k0], t.hw_l2e[s][k1]);
+      }
+  ARGOT_CUDA_TRY(cudaMemcpyToSymbol(d_rate_tab, &rt, sizeof(rt)));
   done[device] = true;
   return 0;
 }
@@ -186,266 +197,238 @@ __device__ __forceinline__ RayParams ray_params_f32(const GridDev &g, int gix, i
   return p;
 }
 
-// The six rates of one ray from its quadrature sums a_s = sum (sigma_s
-// log2 e) w and b_s = sum (sigma_s log2 e) nu w (ray_bins_packed):
-// Gamma_s = P_s ln2 a_s, Heat_s = P_s ln2 (b_s - nu_s a_s) h nu_L.
-__device__ __forceinline__ void ray_rates6(const float (&P)[3], float a0, float a1, float a2, float b0, float b1,
-                                           float b2, float (&out)[6]) {
-  const float kLn2 = 0.69314718055994531f;
-  const float a[3] = {a0, a1, a2}, bb[3] = {b0, b1, b2};
-  const float thr[3] = {(float)kThrHI, (float)kThrHeI, (float)kThrHeII};
-#pragma unroll
-  for (int s = 0; s < 3; s++) {
-    out[s] = P[s] * (kLn2 * a[s]);
-    out[3 + s] = P[s] * (kLn2 * fmaf(-thr[s], a[s], bb[s])) * kHNuLf;
-  }
-}
-
-// ---- packed FP32 bin loop: two bins per instruction with the f32x2 FMA
-// and multiply of sm_100.  An 8-lane group integrates one ray (or two,
-// ray_bins_packed2); lane j owns the bin pairs (j + 16 i, j + 16 i + 8),
-// i = 0..15 (the bins j + 8 m), and keeps one partial sum per output, pair
-// member and ray.
-// The pair table holds, for the three species and the two bins,
-// sigma_s log2(e) and sigma_s log2(e) nu, 48 bytes, three 16-byte shared
-// loads per pair, each serving the two rays of the lane.  The sums run on
-// these entries: sum sigma_s w = ln2 sum (sigma_s log2 e) w, and, because
-// sigma_s vanishes below the species' threshold nu_s (the fits of
-// prim_chem/cross_section.c are 0 there), the heating sum
-// sum sigma_s (nu - nu_s)^+ w = ln2 (sum (sigma_s log2 e) nu w - nu_s
-// sum (sigma_s log2 e) w).  A shared load delivers 128 bytes per wavefront
-// whatever the broadcast (the four groups of a warp read the same
-// entries), so the table's bytes per ray set the kernel's shared-memory
-// traffic, which shares the L1 data path with the spectrum loads.
-// Measured at 256^3 / 4096 sources: with one ray per lane, an 80-byte
-// entry (sigma log2 e, sigma and sigma (nu - nu_s)^+ per species) kept the
-// shared-memory pipe at 79% of its peak, and a 24-byte entry without the
-// nu products (nu formed from the lane's first pair and the grid ratio,
-// two packed multiplies per pair and ray) ran the rates in 0.93 s against
-// 1.02 s for 32 bytes; with two rays per lane this 48-byte entry, which
-// saves those multiplies, runs them in 0.78 s against 0.81 s for 24 bytes.
-struct alignas(16) BinPair {
-  float2 l2e[3];    // sigma_s log2(e) of the two bins
-  float2 l2enu[3];  // sigma_s log2(e) nu
+// ---- FP32 bin loop.  A warp integrates one ray at a time; its lanes share
+// the 256 bins.  Stage m = 0..3 of a ray covers the bins 64 m .. 64 m + 63,
+// lane l the pair (64 m + l, 64 m + l + 32), two bins per instruction with
+// the f32x2 FMA and multiply of sm_100.  A lane's bins are the same for
+// every ray, so their cross sections stay in 44 registers (RateLane) and the
+// spectrum in 8 more until the emitter changes; a ray costs two broadcast
+// shared loads and the reduction of its six sums over the warp.
+// Stage 0 ends below the HeII threshold (bin 102), so it has no HeII terms;
+// they would add exact zeros.
+//
+// What bounds it: the heavy FMA pipe.  A ray takes 62 to 66 packed
+// operations at 2.1 cycles (f32x2 operations issue on that pipe only) and
+// about a dozen scalar ones, 150 cycles of the 205 it takes per SM
+// sub-partition.  Before, four 8-lane groups per warp integrated two rays
+// each and read every bin pair's 48-byte table entry from shared memory and
+// its spectrum from global memory: 145 instructions and 41 L1 data-pipe
+// cycles per ray (63% of that pipe, of which the march beside it needs 77%)
+// against 130 and 23 now.  256^3 cells, 1024 clustered sources, 2.17e9 rays:
+// 0.524 s before, 0.471 s now.  Two rays at a time per warp (for more
+// independent chains): 0.461 s alone, the step with the march no faster.
+struct RateLane {
+  float2 l2e[4][3];  // sigma_s log2(e) of the lane's two bins of each stage
+  float2 h[4][3];    // sigma_s log2(e) (nu - nu_s)^+
 };
-constexpr int kBinPairs = kNu / 2;
-
-// Fills the pair table from the constant tables (all threads of the block
-// take part; the caller synchronises).
-__device__ __forceinline__ void load_bin_pairs(BinPair *tab) {
-  for (int p = threadIdx.x; p < kBinPairs; p += blockDim.x) {
-    const int j = p & 7, i = p >> 3;
-    const int k0 = j + 16 * i, k1 = k0 + 8;
-    BinPair b;
+__device__ __forceinline__ void load_rate_lane(int lane, RateLane &r) {
+#pragma unroll
+  for (int m = 0; m < kStages; m++)
 #pragma unroll
     for (int s = 0; s < 3; s++) {
-      b.l2e[s] = make_float2(c_tab.cs_l2e[s][k0], c_tab.cs_l2e[s][k1]);
-      b.l2enu[s] = make_float2(c_tab.cs_l2e[s][k0] * c_tab.nu_f[k0], c_tab.cs_l2e[s][k1] * c_tab.nu_f[k1]);
+      r.l2e[m][s] = __ldg(&d_rate_tab.v[m][s][lane]);
+      r.h[m][s] = __ldg(&d_rate_tab.v[m][3 + s][lane]);
     }
-    tab[p] = b;
-  }
 }
 
 // The photon-conserving cell factor phi(x) = (1 - e^-x)/x (x the cell's
 // optical depth in the bin) enters every bin as e^-tau phi(x), tau the
 // optical depth to the cell.  Below x = kPhiXMax the difference 1 - e^-x
 // cancels, so the loop forms e^-tau phi(x) = e^-(tau + x/2) sinh(y)/y,
-// y = x / 2, with sinh(y)/y a polynomial (sinhc_half2); above, it takes
-// e^-tau (1 - e^-x) / x from the SFU (~2e-7).  Only the leading iterations
-// of a ray can hold a bin above kPhiXMax (sfu_iters); the SFU form is
-// predicated, not branched, so where it is compiled in every pair pays its
-// exponentials and reciprocal (ncu, 256^3 / 16 sources: three MUFU
-// operations per bin instead of one, 60 warp instructions per iteration
-// instead of ~40), and it is compiled only into those iterations.
+// y = x / 2: the attenuation to the middle of the cell, whose exponent folds
+// into the ray's columns, times an even polynomial; above, it takes
+// e^-tau (1 - e^-x) / x from the SFU (~2e-7).  Below x = kPhiXThin the
+// polynomial is 1 + y^2/6 (the y^4/120 left out is below 7e-9).
 constexpr float kPhiXMax = 1.0f;
 constexpr float kPhiUMax = 1.44269504088896341f;  // kPhiXMax / ln 2
+constexpr float kPhiXThin = 0.06f;
 
 // sinh(y) / y, y = x / 2 = dl ln2 / 2, of the two bins of a pair from
 // v = dl^2: a near-minimax fit of degree 3 in v made by argot_b200/fits.py
 // (fit_sinhc; times the FP32 mid-cell attenuation 2^(-dl/2) it is within
-// 1.5e-7 of phi(x) on [0, 1], checked by the CPU tests).  With it
-// e^-tau phi(x) = e^-(tau + x/2) sinh(y) / y: the attenuation to the middle
-// of the cell, whose exponent folds into the ray's columns, times an even
-// polynomial, one packed multiply and three packed FMAs where the
-// polynomial of phi(x) in x took six FMAs.
+// 1.5e-7 of phi(x) on [0, 1], checked by the CPU tests); thin: its first two
+// terms.
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+template <bool kThin>
 __device__ __forceinline__ float2 sinhc_half2(float2 dl) {
   constexpr float kShc[4] = {1.f, 0.0200188775f, 0.000120223514f, 3.4621803e-07f};
   const float2 v = __fmul2_rn(dl, dl);
-  float2 p = __ffma2_rn(v, make_float2(kShc[3], kShc[3]), make_float2(kShc[2], kShc[2]));
-  p = __ffma2_rn(v, p, make_float2(kShc[1], kShc[1]));
-  return __ffma2_rn(v, p, make_float2(kShc[0], kShc[0]));
+  if (kThin) return __ffma2_rn(v, both(kShc[1]), both(kShc[0]));
+  float2 p = __ffma2_rn(v, both(kShc[3]), both(kShc[2]));
+  p = __ffma2_rn(v, p, both(kShc[1]));
+  return __ffma2_rn(v, p, both(kShc[0]));
 }
 
-// Iterations of ray_bins_packed that may hold a bin with x = sum_s D_s
-// sigma_s(nu) >= kPhiXMax: iteration i covers the bins 16 i .. 16 i + 15,
-// whose x is at most sum_s D_s max_{k >= 16 i} sigma_s (smax16).  That bound
-// does not grow with i, so the iterations that need the SFU path are the
-// leading ones; the rest take the polynomial alone.  (A bin whose x lies
-// within rounding of 1 may take the polynomial, 1e-7 accurate there.)
-__device__ __forceinline__ int sfu_iters(float D0, float D1, float D2) {
-  int n = 0;
+// How the stages of a ray with cell columns D form the factor: 0 thin, 1
+// the degree-3 polynomial, 2 the SFU form for the bins at or above kPhiXMax
+// and the polynomial for the others.  Stage m's x is at most sum_s D_s max
+// sigma_s over its bins and those above (smax).  Four forms of the whole ray
+// are compiled, the cheapest that holds is taken: its stages' forms are
+// 0: 1 0 0 0, 1: 1 1 0 0, 2: 2 1 1 1, 3: 2 2 2 2.  The choice depends on the
+// ray alone, and a ray has the warp to itself, so the branch is uniform.
+__device__ __forceinline__ int ray_form(float D0, float D1, float D2) {
+  int f[kStages];
 #pragma unroll
-  for (int i = 0; i < kNu / 16; i++)
-    n += fmaf(D0, c_tab.smax16[0][i], fmaf(D1, c_tab.smax16[1][i], D2 * c_tab.smax16[2][i])) >= kPhiXMax;
-  return n;
-}
-
-// A ray's columns as the bin loop uses them, each value in both halves of
-// a float2: n = the negated mid-cell columns -(N_s + D_s / 2), d = the
-// cell's columns D_s [cm^-2].
-struct RayCols2 {
-  float2 n[3], d[3];
-};
-__device__ __forceinline__ RayCols2 ray_cols2(float N0, float N1, float N2, float D0, float D1, float D2) {
-  const float N[3] = {N0, N1, N2}, D[3] = {D0, D1, D2};
-  RayCols2 c;
-#pragma unroll
-  for (int q = 0; q < 3; q++) {
-    const float m = -fmaf(0.5f, D[q], N[q]);
-    c.n[q] = make_float2(m, m);
-    c.d[q] = make_float2(D[q], D[q]);
+  for (int m = 0; m < kStages; m++) {
+    const float x = fmaf(D0, c_tab.smax[0][m], fmaf(D1, c_tab.smax[1][m], D2 * c_tab.smax[2][m]));
+    f[m] = x >= kPhiXMax ? 2 : x < kPhiXThin ? 0 : 1;
   }
-  return c;
+  if (max(f[1], max(f[2], f[3])) == 2) return 3;
+  if (f[0] == 2 || f[2] || f[3]) return 2;
+  return f[1];
 }
 
-// One iteration of the bin loop: the bin pair of the lane for one ray.
-// ntm = -(tau + x / 2) log2(e) and w = s 2^ntm sinh(x/2)/(x/2).  With kSfu
-// and `sfu` (an iteration below the ray's own sfu_iters count) a bin with
-// x >= kPhiXMax takes w = s 2^(ntm + dl/2) (1 - 2^-dl) / x instead.  A
-// bin's value depends on its own ray alone, whichever other rays share the
-// loop's round.  kNS: the species whose cross sections can be non-zero in
-// the iteration (1: HI, 2: HI and HeI, 3: all; the others are 0 there and
-// their terms would add exact zeros, so the sums are the same bit for bit).
-template <bool kSfu, int kNS>
-__device__ __forceinline__ void bin_pair(const BinPair &b, float2 s, const RayCols2 &c, float2 (&acc)[6],
-                                         bool sfu = false) {
-  float2 ntm = __fmul2_rn(c.n[kNS - 1], b.l2e[kNS - 1]);
-  float2 dl = __fmul2_rn(c.d[kNS - 1], b.l2e[kNS - 1]);
+// A ray as the loop reads it: n = the negated mid-cell columns
+// -(N_s + D_s / 2), d = the cell's columns D_s [cm^-2], the ray's form, the
+// emitter.
+struct alignas(16) RayRec {
+  float n[3];
+  int form;
+  float d[3];
+  int e;
+};
+__device__ __forceinline__ RayRec ray_rec(const RayParams &p, int e) {
+  RayRec r;
+#pragma unroll
+  for (int s = 0; s < 3; s++) {
+    r.n[s] = -fmaf(0.5f, p.D[s], p.N[s]);
+    r.d[s] = p.D[s];
+  }
+  r.form = ray_form(p.D[0], p.D[1], p.D[2]);
+  r.e = e;
+  return r;
+}
+
+// Stage m of one ray: the lane's two bins.  kNS: species with non-zero cross
+// sections; kForm as in ray_form.  ntm = -(tau + x / 2) log2(e), w = s 2^ntm
+// sinh(x/2)/(x/2) or, with kForm 2 and x >= kPhiXMax, s 2^(ntm + dl/2)
+// (1 - 2^-dl) / x.
+template <int m, int kNS, int kForm>
+__device__ __forceinline__ void rate_stage(const RateLane &t, float2 s, const float2 (&n)[3], const float2 (&d)[3],
+                                           float2 (&acc)[6]) {
+  float2 ntm = __fmul2_rn(n[kNS - 1], t.l2e[m][kNS - 1]);
+  float2 dl = __fmul2_rn(d[kNS - 1], t.l2e[m][kNS - 1]);
 #pragma unroll
   for (int q = kNS - 2; q >= 0; q--) {
-    ntm = __ffma2_rn(c.n[q], b.l2e[q], ntm);
-    dl = __ffma2_rn(c.d[q], b.l2e[q], dl);
+    ntm = __ffma2_rn(n[q], t.l2e[m][q], ntm);
+    dl = __ffma2_rn(d[q], t.l2e[m][q], dl);
   }
   const float2 e = make_float2(ex2_approx(ntm.x), ex2_approx(ntm.y));
-  float2 w = __fmul2_rn(__fmul2_rn(s, e), sinhc_half2(dl));
-  if (kSfu) {
-    const bool t0 = !sfu || dl.x < kPhiUMax, t1 = !sfu || dl.y < kPhiUMax;
-    if (!(t0 && t1)) {
-      const float kLn2 = 0.69314718055994531f;
-      const float2 ntl = __ffma2_rn(dl, make_float2(0.5f, 0.5f), ntm);
-      const float q0 = s.x * ex2_approx(ntl.x) * __fdividef(1.0f - ex2_approx(-dl.x), dl.x * kLn2);
-      const float q1 = s.y * ex2_approx(ntl.y) * __fdividef(1.0f - ex2_approx(-dl.y), dl.y * kLn2);
-      w.x = t0 ? w.x : q0;
-      w.y = t1 ? w.y : q1;
-    }
+  float2 w = __fmul2_rn(__fmul2_rn(s, e), sinhc_half2<kForm == 0>(dl));
+  if (kForm == 2) {
+    const float kLn2 = 0.69314718055994531f;
+    const float2 ntl = __ffma2_rn(dl, both(0.5f), ntm);
+    const float q0 = s.x * ex2_approx(ntl.x) * __fdividef(1.0f - ex2_approx(-dl.x), dl.x * kLn2);
+    const float q1 = s.y * ex2_approx(ntl.y) * __fdividef(1.0f - ex2_approx(-dl.y), dl.y * kLn2);
+    w.x = dl.x < kPhiUMax ? w.x : q0;
+    w.y = dl.y < kPhiUMax ? w.y : q1;
   }
 #pragma unroll
   for (int q = 0; q < kNS; q++) {
-    acc[q] = __ffma2_rn(b.l2e[q], w, acc[q]);
-    acc[3 + q] = __ffma2_rn(b.l2enu[q], w, acc[3 + q]);
+    acc[q] = __ffma2_rn(t.l2e[m][q], w, acc[q]);
+    acc[3 + q] = __ffma2_rn(t.h[m][q], w, acc[3 + q]);
   }
 }
+template <int f0, int f1, int f2, int f3>
+__device__ __forceinline__ void ray_stages(const RateLane &t, const float2 (&sp)[4], const float2 (&n)[3],
+                                           const float2 (&d)[3], float2 (&acc)[6]) {
+  rate_stage<0, 2, f0>(t, sp[0], n, d, acc);
+  rate_stage<1, 3, f1>(t, sp[1], n, d, acc);
+  rate_stage<2, 3, f2>(t, sp[2], n, d, acc);
+  rate_stage<3, 3, f3>(t, sp[3], n, d, acc);
+}
 
-// Unroll factor of the polynomial-only iterations (measured at 256^3 / 4096
-// sources with two rays per lane: at 8 warps x 2 CTAs, 4 runs the rates 2%
-// faster than 2, at 128 registers without spills; at the 96 registers of
-// 5 CTAs of 4 warps, 4 spills and 2 does not).
-#ifndef ARGOT_RATE_UNROLL
-#define ARGOT_RATE_UNROLL 2
-#endif
-constexpr int kRateUnroll = ARGOT_RATE_UNROLL;
-
-// Iterations [i0, i1) of the bin loop for kR rays (1 or 2) of the lane;
-// one load of a table entry serves the kR rays.
-template <int kR, bool kSfu, int kNS>
-__device__ __forceinline__ void bin_iters(const BinPair *__restrict__ tab, const float2 *const (&sp)[kR], int j,
-                                          int i0, int i1, const int (&own)[kR], const RayCols2 (&c)[kR],
-                                          float2 (&acc)[kR][6]) {
-#pragma unroll(kSfu ? 1 : kRateUnroll)
-  for (int i = i0; i < i1; i++) {
-    const BinPair b = tab[j + 8 * i];
-#pragma unroll
-    for (int r = 0; r < kR; r++) bin_pair<kSfu, kNS>(b, __ldg(sp[r] + 8 * i), c[r], acc[r], i < own[r]);
+// The lane's partial sums of one ray: out[s] = (sum (sigma_s log2 e) w, sum
+// (sigma_s log2 e) (nu - nu_s)^+ w) over its bins, w = s_nu e^-tau phi(x).
+// sp: the lane's spectrum of emitter `cur`, read again when the ray's
+// emitter is another one (a block's rays come emitter by emitter).
+__device__ __forceinline__ void ray_bins(const RateLane &t, const RayRec *__restrict__ rec,
+                                         const float *__restrict__ specn, int lane, int &cur, float2 (&sp)[4],
+                                         float2 (&out)[3]) {
+  const float4 ra = *reinterpret_cast<const float4 *>(rec->n), rb = *reinterpret_cast<const float4 *>(rec->d);
+  const int form = __float_as_int(ra.w), e = __float_as_int(rb.w);
+  if (e != cur) {
+    cur = e;
+    const float4 *p = reinterpret_cast<const float4 *>(specn + (size_t)e * kNu) + 2 * lane;
+    const float4 a = __ldg(p), b = __ldg(p + 1);
+    sp[0] = make_float2(a.x, a.y);
+    sp[1] = make_float2(a.z, a.w);
+    sp[2] = make_float2(b.x, b.y);
+    sp[3] = make_float2(b.z, b.w);
   }
+  const float2 n[3] = {both(ra.x), both(ra.y), both(ra.z)}, d[3] = {both(rb.x), both(rb.y), both(rb.z)};
+  float2 acc[6];
+#pragma unroll
+  for (int q = 0; q < 6; q++) acc[q] = both(0.f);
+  if (form == 0) ray_stages<1, 0, 0, 0>(t, sp, n, d, acc);
+  else if (form == 1) ray_stages<1, 1, 0, 0>(t, sp, n, d, acc);
+  else if (form == 2) ray_stages<2, 1, 1, 1>(t, sp, n, d, acc);
+  else ray_stages<2, 2, 2, 2>(t, sp, n, d, acc);
+#pragma unroll
+  for (int q = 0; q < 3; q++) out[q] = make_float2(acc[q].x + acc[q].y, acc[3 + q].x + acc[3 + q].y);
 }
 
-// The lane's six partial sums of kR rays (1 or 2) from the columns c; sp:
-// the emitters' normalised spectra as bin pairs, offset to the lane; j: the
-// lane in the rays' 8-lane group; the first nsfu iterations are compiled
-// with the SFU form (the caller passes the same count, the round's largest
-// sfu_iters, to the four groups of the warp, so that their loops stay
-// converged), which a ray takes in its own first own[r] (its sfu_iters);
-// the loop runs in three stretches by the species present (iter_he,
-// iter_heii of the tables), in increasing iteration order:
-// out[r][s] = sum (sigma_s log2 e) w, out[r][3 + s] = sum (sigma_s log2 e)
-// nu w over the lane's bins, w = s_nu e^-tau phi(dtau).  The caller adds the
-// eight lanes and forms the rates (ray_rates6).
-template <int kR>
-__device__ __forceinline__ void ray_bins(const BinPair *__restrict__ tab, const float2 *const (&sp)[kR], int j,
-                                         int nsfu, const int (&own)[kR], const RayCols2 (&c)[kR],
-                                         float (&out)[kR][6]) {
-  float2 acc[kR][6];
-#pragma unroll
-  for (int r = 0; r < kR; r++)
-#pragma unroll
-    for (int q = 0; q < 6; q++) acc[r][q] = make_float2(0.f, 0.f);
-  constexpr int kIters = kBinPairs / 8;
-  const int h1 = c_tab.iter_he, h2 = c_tab.iter_heii;
-  const int s1 = min(nsfu, h1), s2 = min(max(nsfu, h1), h2), s3 = max(nsfu, h2);
-  bin_iters<kR, true, 1>(tab, sp, j, 0, s1, own, c, acc);
-  bin_iters<kR, false, 1>(tab, sp, j, s1, h1, own, c, acc);
-  bin_iters<kR, true, 2>(tab, sp, j, h1, s2, own, c, acc);
-  bin_iters<kR, false, 2>(tab, sp, j, s2, h2, own, c, acc);
-  bin_iters<kR, true, 3>(tab, sp, j, h2, min(s3, kIters), own, c, acc);
-  bin_iters<kR, false, 3>(tab, sp, j, s3, kIters, own, c, acc);
-#pragma unroll
-  for (int r = 0; r < kR; r++)
-#pragma unroll
-    for (int q = 0; q < 6; q++) out[r][q] = acc[r][q].x + acc[r][q].y;
-}
+// Per-warp scratch of the FP32 rates: a chunk of 32 rays.
+constexpr int kRoundRays = 4;
+constexpr int kRedRow = 34;  // float2 per row: 16-byte reads of 8 rows fall on different banks
+struct RateChunk {
+  RayRec rec[32];
+  float2 red[3 * kRoundRays][kRedRow];  // a round's lane sums, row 3 k + s: ray k, species s
+  float p[32][3];    // prefactors P_s
+  float out[32][6];  // per-ray rates
+};
 
-// One ray: columns N (to the cell) and D (of the cell) in cm^-2, sp the
-// emitter's normalised spectrum.
-__device__ __forceinline__ void ray_bins_packed(const BinPair *__restrict__ tab, const float *__restrict__ sp,
-                                                int j, int nsfu, int own, float N0, float N1, float N2, float D0,
-                                                float D1, float D2, float (&out)[6]) {
-  // the pair's two spectrum bins in one 8-byte load (pair order)
-  const float2 *const sp2[1] = {reinterpret_cast<const float2 *>(sp) + j};
-  const int own1[1] = {own};
-  const RayCols2 c[1] = {ray_cols2(N0, N1, N2, D0, D1, D2)};
-  float o[1][6];
-  ray_bins<1>(tab, sp2, j, nsfu, own1, c, o);
+// The rates of nq rays of a chunk (ray i is entry q[i], or i without q):
+// S.out[ray] = Gamma_s = P_s ln2 a_s, Heat_s = P_s ln2 b_s h nu_L.  All lanes
+// of the warp take part; the caller synchronises the warp before and after.
+// Rounds of kRoundRays rays: every lane leaves its three pairs of sums per
+// ray in shared memory, then lane r and lane r + 16 add the lanes 0..15 and
+// 16..31 of row r (a butterfly over the warp takes 60 instructions per ray,
+// a recursive halving 25, this 10).
+__device__ __forceinline__ void chunk_rates(RateChunk &S, const RateLane &t, const float *__restrict__ specn,
+                                            const int *q, int nq, int lane) {
+  const float kLn2 = 0.69314718055994531f;
+  const int row = lane & 15, kr = row / 3, s = row - 3 * kr;
+  float2 sp[4];
+  int cur = -1;
+  for (int i = 0; i < nq; i += kRoundRays) {
+    const int nr = min(kRoundRays, nq - i);
+#pragma unroll 1
+    for (int k = 0; k < nr; k++) {
+      float2 o[3];
+      ray_bins(t, &S.rec[q ? q[i + k] : i + k], specn, lane, cur, sp, o);
 #pragma unroll
-  for (int q = 0; q < 6; q++) out[q] = o[0][q];
-}
-
-// Two rays (columns nd = N0, N1, N2, D0, D1, D2 of each, own SFU counts
-// owna, ownb): one load of each bin pair of the table serves both rays,
-// which halves the shared-memory traffic per ray; nsfu covers both.
-__device__ __forceinline__ void ray_bins_packed2(const BinPair *__restrict__ tab, const float *__restrict__ spa,
-                                                 const float *__restrict__ spb, int j, int nsfu, int owna,
-                                                 int ownb, const float *nda, const float *ndb, float (&outa)[6],
-                                                 float (&outb)[6]) {
-  const float2 *const sp2[2] = {reinterpret_cast<const float2 *>(spa) + j, reinterpret_cast<const float2 *>(spb) + j};
-  const int own[2] = {owna, ownb};
-  const RayCols2 c[2] = {ray_cols2(nda[0], nda[1], nda[2], nda[3], nda[4], nda[5]),
-                         ray_cols2(ndb[0], ndb[1], ndb[2], ndb[3], ndb[4], ndb[5])};
-  float o[2][6];
-  ray_bins<2>(tab, sp2, j, nsfu, own, c, o);
+      for (int c = 0; c < 3; c++) S.red[3 * k + c][lane] = o[c];
+    }
+    __syncwarp();
+    float2 sum = both(0.f);
+    if (kr < nr) {
+      const float4 *p = reinterpret_cast<const float4 *>(&S.red[row][lane & 16]);
+      float4 v[8];
 #pragma unroll
-  for (int q = 0; q < 6; q++) {
-    outa[q] = o[0][q];
-    outb[q] = o[1][q];
+      for (int c = 0; c < 8; c++) v[c] = p[c];
+#pragma unroll
+      for (int o = 4; o; o >>= 1)
+#pragma unroll
+        for (int c = 0; c < o; c++)
+          v[c] = make_float4(v[c].x + v[c + o].x, v[c].y + v[c + o].y, v[c].z + v[c + o].z, v[c].w + v[c + o].w);
+      sum = make_float2(v[0].x + v[0].z, v[0].y + v[0].w);
+    }
+    sum.x += __shfl_xor_sync(0xffffffffu, sum.x, 16);
+    sum.y += __shfl_xor_sync(0xffffffffu, sum.y, 16);
+    if (kr < nr && lane < 16) {
+      const int ray = q ? q[i + kr] : i + kr;
+      const float P = S.p[ray][s];
+      S.out[ray][s] = P * (kLn2 * sum.x);
+      S.out[ray][3 + s] = P * (kLn2 * sum.y) * kHNuLf;
+    }
+    __syncwarp();
   }
 }
 
 // Per-warp scratch of rate_block_f32.
 struct RateWarpSmem {
-  float nd[32][6];   // N_s, D_s of the chunk's rays (cm^-2)
-  float p[32][3];    // prefactors P_s
-  float out[32][6];  // per-ray rates
-  int e[32], t[32];  // emitter, target lane
-  int nsfu[32];      // iterations of the bin loop that may need the SFU path (sfu_iters)
+  RateChunk c;
   float acc[12][32]; // per target lane: Kahan sums and compensations (CellSum6Smem)
   int q[32];         // lanes of the chunk's rays that take the quadrature
   int cnt[32], src[32];  // per target lane: rays of the chunk, ray of the round
@@ -515,24 +498,21 @@ __device__ __forceinline__ void add_chunk_in_order(Acc &acc, int lane, int t, co
 // The FP32 rates of one target block b whose rays are [r0, r1) of `rays`
 // (columns in three planes of nray), written to its cells in rates6; one
 // warp.  Phase A: per-ray parameters (ray_params_f32), one lane per ray, 32
-// rays at a time.  Phase B: four 8-lane groups, one ray each, over the bin
-// pairs (ray_bins_packed; with kRaysPerLane 2, two rays per group,
-// ray_bins_packed2), three butterfly steps.  Phase C: lane j adds the
-// rays of cell j of the block in ray order (add_chunk_in_order).
+// rays at a time.  Phase B: the chunk's rays one after another
+// (chunk_rates).  Phase C: lane j adds the rays of cell j of the block in
+// ray order (add_chunk_in_order).
 // kServed: `pred` holds 7 planes of nray floats, six per-ray contributions
 // and a flag; a ray whose flag is non-zero contributes those six values
 // and skips the quadrature, which runs over the remaining rays of the
 // chunk only (the surrogate's fallback).
-template <bool kServed = false, int kRaysPerLane = 1>
+template <bool kServed = false>
 __device__ __forceinline__ void rate_block_f32(const GridDev &g, const float4 *__restrict__ raw,
                                                const float4 *__restrict__ emit_pos, const float *__restrict__ specn,
-                                               const double *__restrict__ total, const BinPair *__restrict__ pairs,
+                                               const double *__restrict__ total, const RateLane &tab,
                                                uint64_t b, uint64_t r0, uint64_t r1,
                                                const uint32_t *__restrict__ rays, uint64_t nray,
                                                const float *__restrict__ tau, float *__restrict__ rates6,
                                                RateWarpSmem &S, int lane, const float *__restrict__ pred = nullptr) {
-  const int grp = lane >> 3, j = lane & 7;
-  const unsigned gmask = 0xffu << (8 * grp);
   const uint64_t ncell = (uint64_t)g.nx * g.ny * g.nz;
   int ix, iy, iz;
   const bool own_valid = block_cell(g, b, lane, &ix, &iy, &iz);
@@ -551,7 +531,7 @@ __device__ __forceinline__ void rate_block_f32(const GridDev &g, const float4 *_
       t = (int)(w & 31u);
       if (kServed && __ldg(pred + 6 * nray + r) != 0.f) {
 #pragma unroll
-        for (int s = 0; s < 6; s++) S.out[lane][s] = __ldg(pred + s * nray + r);
+        for (int s = 0; s < 6; s++) S.c.out[lane][s] = __ldg(pred + s * nray + r);
       } else {
         quad = true;
         const int lx = bix + (t >> 4), ly = biy + ((t >> 2) & 3), lz = biz + (t & 3);
@@ -559,90 +539,21 @@ __device__ __forceinline__ void rate_block_f32(const GridDev &g, const float4 *_
         const float4 rw = __ldg(raw + cell_index(g, lx, ly, lz));
         const RayParams p = ray_params_f32(g, g.ix0 + lx, g.iy0 + ly, g.iz0 + lz, ep.x, ep.y, ep.z, __ldg(tau + r),
                                            __ldg(tau + nray + r), __ldg(tau + 2 * nray + r), rw, __ldg(total + e));
+        S.c.rec[lane] = ray_rec(p, (int)e);
 #pragma unroll
-        for (int s = 0; s < 3; s++) {
-          S.nd[lane][s] = p.N[s];
-          S.nd[lane][3 + s] = p.D[s];
-          S.p[lane][s] = p.P[s];
-        }
-        S.e[lane] = (int)e;
-        S.nsfu[lane] = sfu_iters(p.D[0], p.D[1], p.D[2]);
+        for (int s = 0; s < 3; s++) S.c.p[lane][s] = p.P[s];
       }
     }
-    S.t[lane] = t;
-    const int nk = (int)min((uint64_t)32, r1 - rc);
-    int nq = nk;
+    int nq = (int)min((uint64_t)32, r1 - rc);
     if (kServed) {
       const unsigned m = __ballot_sync(0xffffffffu, quad);
       if (quad) S.q[__popc(m & ((1u << lane) - 1u))] = lane;
       nq = __popc(m);
     }
     __syncwarp();
-    // rounds of four (eight) rays, one (two) per group; the groups of a
-    // round run the same bin loop (the largest SFU count of the round), so
-    // that the warp stays converged; a group without a ray in the last
-    // round repeats the round's first ray and discards it
-    static_assert(kRaysPerLane == 1 || kRaysPerLane == 2, "one or two rays per lane");
-    if constexpr (kRaysPerLane == 2) {
-      for (int i0 = 0; i0 < nq; i0 += 8) {
-        const int ia = i0 + grp < nq ? i0 + grp : i0, ib = i0 + 4 + grp < nq ? i0 + 4 + grp : i0;
-        const int qa = kServed ? S.q[ia] : ia, qb = kServed ? S.q[ib] : ib;
-        int nsfu = 0;
-#pragma unroll
-        for (int k = 0; k < 8; k++) nsfu = max(nsfu, i0 + k < nq ? S.nsfu[kServed ? S.q[i0 + k] : i0 + k] : 0);
-        float pa[6], pb[6];
-        ray_bins_packed2(pairs, specn + (size_t)S.e[qa] * kNu, specn + (size_t)S.e[qb] * kNu, j, nsfu, S.nsfu[qa],
-                         S.nsfu[qb], S.nd[qa], S.nd[qb], pa, pb);
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) {
-#pragma unroll
-          for (int s = 0; s < 6; s++) {
-            pa[s] += __shfl_xor_sync(gmask, pa[s], o);
-            pb[s] += __shfl_xor_sync(gmask, pb[s], o);
-          }
-        }
-        if (j == 0) {
-          float out[6];
-          if (i0 + grp < nq) {
-            const float P[3] = {S.p[qa][0], S.p[qa][1], S.p[qa][2]};
-            ray_rates6(P, pa[0], pa[1], pa[2], pa[3], pa[4], pa[5], out);
-#pragma unroll
-            for (int s = 0; s < 6; s++) S.out[qa][s] = out[s];
-          }
-          if (i0 + 4 + grp < nq) {
-            const float P[3] = {S.p[qb][0], S.p[qb][1], S.p[qb][2]};
-            ray_rates6(P, pb[0], pb[1], pb[2], pb[3], pb[4], pb[5], out);
-#pragma unroll
-            for (int s = 0; s < 6; s++) S.out[qb][s] = out[s];
-          }
-        }
-      }
-    } else {
-      for (int i0 = 0; i0 < nq; i0 += 4) {
-        const int i = i0 + grp < nq ? i0 + grp : i0;
-        const int q = kServed ? S.q[i] : i;
-        int nsfu = 0;
-#pragma unroll
-        for (int k = 0; k < 4; k++) nsfu = max(nsfu, i0 + k < nq ? S.nsfu[kServed ? S.q[i0 + k] : i0 + k] : 0);
-        float part[6];
-        ray_bins_packed(pairs, specn + (size_t)S.e[q] * kNu, j, nsfu, S.nsfu[q], S.nd[q][0], S.nd[q][1], S.nd[q][2],
-                        S.nd[q][3], S.nd[q][4], S.nd[q][5], part);
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) {
-#pragma unroll
-          for (int s = 0; s < 6; s++) part[s] += __shfl_xor_sync(gmask, part[s], o);
-        }
-        if (j == 0 && i0 + grp < nq) {
-          const float P[3] = {S.p[q][0], S.p[q][1], S.p[q][2]};
-          float out[6];
-          ray_rates6(P, part[0], part[1], part[2], part[3], part[4], part[5], out);
-#pragma unroll
-          for (int s = 0; s < 6; s++) S.out[q][s] = out[s];
-        }
-      }
-    }
+    chunk_rates(S.c, tab, specn, kServed ? S.q : nullptr, nq, lane);
     __syncwarp();
-    add_chunk_in_order(acc, lane, t, S.out, S.cnt, S.src);
+    add_chunk_in_order(acc, lane, t, S.c.out, S.cnt, S.src);
   }
   if (own_valid) {
 #pragma unroll

@@ -243,7 +243,7 @@ __global__ void k_emitters(int nn, int n, const DevNode *__restrict__ nodes, con
   __syncthreads();
   const double inv = tot > 0.0 ? __ddiv_rn(1.0, tot) : 0.0;
   for (int b = threadIdx.x; b < kNu; b += blockDim.x)
-    especn[(size_t)e * kNu + spec_pair_index(b)] = __double2float_rn(__dmul_rn(s[b], inv));
+    especn[(size_t)e * kNu + spec_lane_index(b)] = __double2float_rn(__dmul_rn(s[b], inv));
 }
 
 // bounding box of the emitter positions (one block)

@@ -128,3 +128,27 @@ def test_overlapped_run_equals_sequential(cuda_ok):
     torch.cuda.synchronize()
     assert torch.equal(got, want) and int(cnt.item()) > 0
     pb.check_device_error()
+
+
+@pytest.mark.parametrize("edge,nsrc", [(4, 1), (5, 2), (7, 3), (8, 5)])
+@pytest.mark.parametrize("scale", [1e-4, 0.05, 0.5, 2.0, 30.0, 1e3])
+def test_f32_forms_and_partial_rounds(cuda_ok, edge, nsrc, scale):
+    """The FP32 loop's forms of the cell factor (thin cells to cells of
+    optical depth far above 1) and its partial rounds (chunks of 1 to 32
+    rays), against the FP64 rates of the same columns.  The FP32 exponent
+    carries a few 2^-24 of tau, and the bins that make up a rate have tau
+    below about 20: 1e-5."""
+    from argot_b200 import _lib as L, workload as W
+    from argot_b200.pipeline import Problem
+    wl = W.plain(edge, nsrc, seed=edge)
+    wl.dens = (wl.dens * np.float32(scale * 64 / edge)).astype(np.float32)
+    out = []
+    for mode in (L.RATE_EXACT_F64, L.RATE_EXACT_F32):
+        pb = Problem(wl)
+        r = pb.run(L.PRECISION_KAHAN, mode)
+        pb.check_device_error()
+        out.append(r.view(6, -1).double().cpu().numpy())
+    f64, f32 = out
+    big = f64 > 1e-30 * f64.max(axis=1, keepdims=True)
+    assert big.any(axis=1).all()
+    assert (np.abs(f32 - f64)[big] / f64[big]).max() < 1e-5

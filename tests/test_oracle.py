@@ -225,3 +225,18 @@ def test_mid_cell_polynomial_matches_fit_and_bound():
     lhs = np.exp(-tau) * fits.phi(x)
     rhs = np.exp(-(tau + x / 2)) * fits.sinhc_half(x / fits.LN2)
     assert np.max(np.abs(lhs - rhs) / lhs) < 1e-14
+
+
+def test_thin_form_of_the_cell_factor():
+    """Below x = kPhiXThin the FP32 rate kernel keeps the first two terms of
+    the sinh(y)/y polynomial: what it leaves out, y^4/120 and the fit's
+    difference from 1/6, stays below a quarter of an FP32 ulp."""
+    import os
+    import re
+    from argot_b200 import fits
+    from conftest import ROOT
+    src = open(os.path.join(ROOT, "argot_b200", "csrc", "photoion.cuh")).read()
+    thin = float(re.search(r"kPhiXThin\s*=\s*([0-9.]+)f", src).group(1))
+    c1 = float(fits.fit_sinhc()[1])
+    u = np.linspace(0.0, thin / fits.LN2, 2001)
+    assert np.max(np.abs(1.0 + c1 * u * u - fits.sinhc_half(u))) < 2.0 ** -26
