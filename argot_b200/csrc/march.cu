@@ -3,6 +3,8 @@
 // (accum_optical_depth) on sm_100a.
 #include <cub/device/device_scan.cuh>
 
+#include <algorithm>
+
 #include "march.cuh"
 
 namespace argot {
@@ -134,33 +136,77 @@ __global__ void __launch_bounds__(256) k_walk(GridDev g, const DevNode *__restri
 // Consecutive rays of a block come from the same emitter and end in
 // neighbouring cells, so the 32 lanes march nearly parallel paths of nearly
 // equal length and their gathers hit the same cache lines.
-// Launch shape: 256 threads, at least ARGOT_MARCH_MIN_CTAS CTAs resident per
-// SM (which caps the registers per thread).  The march is bound by the
-// latency of its cache-hit gathers, so resident warps matter more than
-// registers: measured on B200 at 256^3 / 4096 sources with the fixed-point
-// walk, 8 CTAs (32 registers) 1.15 s, 7 CTAs 1.15 s, 6 CTAs (40 registers)
-// 1.21 s.  What lives across a ray's walk is kept out of registers: the
-// Kahan columns in per-thread shared-memory slots, the block's state (block
-// index, ray count, packed coordinates, first ray; the same for the warp's
-// lanes) in per-warp shared memory, read back after each ray.  That took the
-// 8-CTA launch from 1.76 s (spilling) to 1.15 s.  kInside: every emitter
-// lies inside the box (the host checks the emitters' bounding box), so rays
-// start at their emitter and the launch contains no call.
-#ifndef ARGOT_MARCH_MIN_CTAS
-#define ARGOT_MARCH_MIN_CTAS 8
-#endif
-#ifndef ARGOT_MARCH_CENTRE_END
-#define ARGOT_MARCH_CENTRE_END true
-#endif
-// CTA size (measured at 256^3 / 4096 sources: 128 threads x 16 CTAs run the
-// march alone 5% faster than 256 x 8, but the step that overlaps it with
-// the rates 0.6% slower).
-#ifndef ARGOT_MARCH_THREADS
-#define ARGOT_MARCH_THREADS 256
-#endif
-constexpr int kMarchThreads = ARGOT_MARCH_THREADS;
-template <int kPrec, bool kInside>
-__global__ void __launch_bounds__(kMarchThreads, ARGOT_MARCH_MIN_CTAS) k_march_rays(GridDev g, const float4 *__restrict__ cells,
+//
+// Which blocks run at the same time decides where the gathers hit: warps
+// work through their emitters in the same depth-first order, so blocks that
+// lie together walk the same cells.  Blocks are therefore taken in tiles
+// (block_of_item): the 32 warps of a CTA hold 2 x 4 x 4 blocks (4 x 16 x 16
+// cells), consecutive CTAs 8 x 8 x 8 blocks, instead of a row of blocks along
+// z.  ncu, 224^3 cells / 32 sources: L1 sector hits 37% -> 56%, L2 63% -> 89%,
+// DRAM no longer read 64 GB per launch, 82.9 -> 72.5 ms; 256^3 / 1024
+// clustered sources: 0.697 s -> 0.610 s (CTAs of 8 warps in tiles 0.664 s, of
+// 16 warps 0.629 s).  What bounds it now: the L1 data pipe (77% of its peak,
+// one line per cycle for each quarter warp of a 16-byte gather), the ALU
+// (68%) and issue (71%) together.
+// Launch shape: 64 warps per SM (32 registers) in CTAs of 32 warps; a range
+// of blocks that would leave SMs empty that way (fewer than kWideBlocks)
+// takes CTAs of 8 warps.  What lives across a ray's walk is kept out of
+// registers: the Kahan columns in per-thread shared-memory slots, the
+// block's state (item, ray count, packed coordinates, first ray; the same
+// for the warp's lanes) in per-warp shared memory, read back after each ray.
+// kInside: every emitter lies inside the box (the host checks the emitters'
+// bounding box), so rays start at their emitter and the launch contains no
+// call.
+constexpr int kMarchWide = 1024, kMarchNarrow = 256;
+constexpr uint64_t kWideBlocks = 148 * 64;
+
+// One level of a tiled enumeration of nx * ny * nz blocks (tiles of tx * ty *
+// tz, those at the high ends clipped; tiles in (x, y, z) order with z
+// fastest): the origin and extents of the tile that holds item i and the
+// item's rank r in it.
+struct TileAt {
+  uint32_t x, y, z, nx, ny, nz, r;
+};
+__device__ __forceinline__ TileAt tile_at(uint32_t i, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t tx, uint32_t ty,
+                                          uint32_t tz) {
+  TileAt t;
+  const uint32_t a = i / (tx * ny * nz);
+  i -= a * (tx * ny * nz);
+  t.x = a * tx;
+  t.nx = min(tx, nx - t.x);
+  const uint32_t b = i / (t.nx * ty * nz);
+  i -= b * (t.nx * ty * nz);
+  t.y = b * ty;
+  t.ny = min(ty, ny - t.y);
+  const uint32_t c = i / (t.nx * t.ny * tz);
+  t.z = c * tz;
+  t.nz = min(tz, nz - t.z);
+  t.r = i - c * (t.nx * t.ny * tz);
+  return t;
+}
+
+// The block that item `it` of the range [b0, b1) stands for: the whole
+// x-slabs of blocks in the range in tiles of 8 x 8 x 8 blocks and, within
+// them, of 2 x 4 x 4; the blocks of a partial slab at either end as they are.
+// A permutation of the range.
+__device__ __forceinline__ uint32_t block_of_item(uint32_t nby, uint32_t nbz, uint32_t it, uint32_t b0, uint32_t b1) {
+  const uint32_t nyz = nby * nbz, x0 = (b0 + nyz - 1) / nyz, x1 = b1 / nyz;
+  if (x1 <= x0 || it < x0 * nyz || it >= x1 * nyz) return it;
+  const TileAt t = tile_at(it - x0 * nyz, x1 - x0, nby, nbz, 8, 8, 8);
+  const TileAt u = tile_at(t.r, t.nx, t.ny, t.nz, 2, 4, 4);
+  const uint32_t dx = u.r / (u.ny * u.nz), yz = u.r - dx * (u.ny * u.nz), dy = yz / u.nz, dz = yz - dy * u.nz;
+  return ((x0 + t.x + u.x + dx) * nby + (t.y + u.y + dy)) * nbz + (t.z + u.z + dz);
+}
+
+// The ray of a chunk of 32 that a lane takes: 8 consecutive lanes, which a
+// 16-byte gather serves together, take 2 x 2 x 2 neighbouring cells (8% fewer
+// lines per gather than 2 rows of 4).
+__device__ __forceinline__ uint32_t chunk_ray(uint32_t lane) {
+  return ((lane & 4u) << 2) | ((lane & 16u) >> 1) | ((lane & 2u) << 1) | ((lane & 8u) >> 2) | (lane & 1u);
+}
+
+template <int kPrec, bool kInside, int kThreads>
+__global__ void __launch_bounds__(kThreads, 2048 / kThreads) k_march_rays(GridDev g, const float4 *__restrict__ cells,
                                                     const float4 *__restrict__ emit_pos, uint32_t b0,
                                                     uint32_t b1, const uint64_t *__restrict__ blk_off,
                                                     uint64_t base, const uint32_t *__restrict__ rays,
@@ -170,14 +216,15 @@ __global__ void __launch_bounds__(kMarchThreads, ARGOT_MARCH_MIN_CTAS) k_march_r
   const int lane = threadIdx.x & 31;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarp = (gridDim.x * blockDim.x) >> 5;
-  __shared__ float kslot[6 * kMarchThreads];  // the Kahan columns, one slot per thread
+  __shared__ float kslot[6 * kThreads];  // the Kahan columns, one slot per thread
   // the block's state, the same for the warp's lanes: it is read back from
   // shared memory after each ray instead of staying live in registers
-  // across the walk (block index, ray count, packed coordinates, first ray)
-  __shared__ uint32_t wstate[kMarchThreads / 32][5];
+  // across the walk (item, ray count, packed coordinates, first ray)
+  __shared__ uint32_t wstate[kThreads / 32][5];
   volatile uint32_t *ws = wstate[threadIdx.x >> 5];
   bool bad = false;
-  for (uint32_t b = b0 + warp; b < b1; b += nwarp) {
+  for (uint32_t it = b0 + warp; it < b1; it += nwarp) {
+    const uint32_t b = block_of_item((uint32_t)g.nby, (uint32_t)g.nbz, it, b0, b1);
     uint64_t r0, r1;
     if (!block_rays(blk_off, b, base, nray, &r0, &r1)) { bad = true; continue; }
     // the block's coordinates in blocks (the host checks nbx < 4096 and
@@ -186,7 +233,7 @@ __global__ void __launch_bounds__(kMarchThreads, ARGOT_MARCH_MIN_CTAS) k_march_r
     const uint32_t bx = b / nyz, by = (b - bx * nyz) / (uint32_t)g.nbz, bz = b - bx * nyz - by * (uint32_t)g.nbz;
     __syncwarp();
     if (lane == 0) {
-      ws[0] = b;
+      ws[0] = it;
       ws[1] = (uint32_t)(r1 - r0);
       ws[2] = bx | (by << 12) | (bz << 22);
       ws[3] = (uint32_t)r0;
@@ -194,7 +241,7 @@ __global__ void __launch_bounds__(kMarchThreads, ARGOT_MARCH_MIN_CTAS) k_march_r
     }
     __syncwarp();
     uint32_t bsteps = 0;
-    for (uint32_t j = lane; j < ws[1]; j += 32) {
+    for (uint32_t j = chunk_ray(lane); j < ws[1]; j += 32) {
       const uint64_t r = (((uint64_t)ws[4] << 32) | ws[3]) + j;
       const uint32_t bpos = ws[2];
       const uint32_t w = __ldg(rays + r);
@@ -212,8 +259,8 @@ __global__ void __launch_bounds__(kMarchThreads, ARGOT_MARCH_MIN_CTAS) k_march_r
       int steps = 0;
       const Tau3 t = (kPrec == ARGOT_B200_PRECISION_REFERENCE)
                          ? march_reference(g, cells, xs, ys, zs, xe, ye, ze, &steps, &bad)
-                         : march_kahan<kMarchThreads, ARGOT_MARCH_CENTRE_END>(g, cells, xs, ys, zs, xe, ye, ze,
-                                                                              &steps, &bad, kslot + threadIdx.x);
+                         : march_kahan<kThreads, true>(g, cells, xs, ys, zs, xe, ye, ze, &steps, &bad,
+                                                       kslot + threadIdx.x);
       const uint64_t ro = (((uint64_t)ws[4] << 32) | ws[3]) + j;
       tau[ro] = t.hi;
       tau[nray + ro] = t.hei;
@@ -224,7 +271,7 @@ __global__ void __launch_bounds__(kMarchThreads, ARGOT_MARCH_MIN_CTAS) k_march_r
       for (int o = 16; o; o >>= 1) bsteps += __shfl_xor_sync(0xffffffffu, bsteps, o);
       if (lane == 0 && bsteps) atomicAdd(crossings, (unsigned long long)bsteps);
     }
-    b = ws[0];
+    it = ws[0];
   }
   if (bad) atomicExch(err, 1);
 }
@@ -436,14 +483,16 @@ int argot_b200_march_rays(const argot_b200_grid *gp, const void *packed, const a
   int *err = err_flag(dev);
   if (!err) { set_status(ARGOT_B200_ENOMEM); return ARGOT_B200_ENOMEM; }
   cudaStream_t st = (cudaStream_t)stream;
-  const int threads = kMarchThreads;
+  const bool wide = b1 - b0 >= kWideBlocks;
+  const int threads = wide ? kMarchWide : kMarchNarrow;
   const int blocks = grid_blocks_for((b1 - b0) * 32, threads);
   const bool inside = t->emit_lo[0] >= gp->xmin && t->emit_lo[1] >= gp->ymin && t->emit_lo[2] >= gp->zmin &&
                       t->emit_hi[0] <= gp->xmax && t->emit_hi[1] <= gp->ymax && t->emit_hi[2] <= gp->zmax;
   const float4 *cells = (const float4 *)packed;
-#define ARGOT_MARCH_LAUNCH(P, I)                                                                       \
-  k_march_rays<P, I><<<blocks, threads, 0, st>>>(g, cells, t->emit_pos, (uint32_t)b0, (uint32_t)b1, blk_off, \
-                                                 base, rays, nray, tau, crossings, err)
+#define ARGOT_MARCH_LAUNCH(P, I)                                                            \
+  (wide ? k_march_rays<P, I, kMarchWide> : k_march_rays<P, I, kMarchNarrow>)                \
+      <<<blocks, threads, 0, st>>>(g, cells, t->emit_pos, (uint32_t)b0, (uint32_t)b1,       \
+                                   blk_off, base, rays, nray, tau, crossings, err)
   if (prec == ARGOT_B200_PRECISION_REFERENCE) {
     if (inside) ARGOT_MARCH_LAUNCH(ARGOT_B200_PRECISION_REFERENCE, true);
     else ARGOT_MARCH_LAUNCH(ARGOT_B200_PRECISION_REFERENCE, false);

@@ -259,3 +259,32 @@ def test_stitch_flags_ray_index_past_the_rays(cuda_ok):
     got = out.cpu().numpy()
     assert np.array_equal(got[:nray], np.ones((nray, 3), np.float32))
     assert not got[nray:].any()
+
+
+@pytest.mark.parametrize("edge,nsrc", [(3, 2), (10, 3), (19, 5), (33, 2), (70, 1), (75, 2)])
+def test_block_order_covers_every_range(cuda_ok, edge, nsrc):
+    """The march takes its blocks in tiles: every ray of a block range (whole
+    slabs, partial slabs at either end, a few blocks) is marched once, with
+    the columns of the whole range."""
+    import torch
+    from argot_b200 import _lib as L, workload as W
+    from argot_b200.pipeline import Problem, RayGroup
+    pb = Problem(W.plain(edge, nsrc, seed=edge))
+    g = pb.groups[0]
+    rays, tau = pb.alloc_group_buffers()
+    pb.emit(g, rays)
+    for prec in (L.PRECISION_KAHAN, L.PRECISION_REFERENCE):
+        tau.fill_(float("nan"))
+        pb.march(g, rays, tau, prec)
+        whole = tau.view(3, -1).clone()
+        assert not torch.isnan(whole).any()
+        nb, slab = pb.nblocks, ((edge + 3) // 4) ** 2
+        for b0, b1 in ((0, nb - 1), (1, nb), (slab // 2, nb - slab // 3), (nb // 3, nb // 3 + 2), (nb - 1, nb)):
+            lo, hi = int(pb.blk_off_host[b0]), int(pb.blk_off_host[b1])
+            n = hi - lo
+            if n < 1:
+                continue
+            part = torch.full((3 * n,), float("nan"), device="cuda")
+            pb.march(RayGroup(b0, b1, lo, n), rays[lo:], part, prec)
+            assert torch.equal(part.view(3, n), whole[:, lo:hi])
+    pb.check_device_error()
