@@ -16,15 +16,19 @@
 // (HI, HeI, HeII edges), I (1 - e^-tau) and the chord length to the angle's
 // accumulators, and updates I = I e^-tau + S (1 - e^-tau).
 //
-// B200 design.  A pass takes a batch of angles: one thread per ray, all
-// rays of all angles of the batch in one launch (a single angle has only
-// N^2 rays), each angle with its own accumulator planes, so the per-angle
-// sums stay separate as the reference needs them.  Rays of one angle are
-// parallel lines, several may cross a cell, so the accumulators take vector
-// float atomics (one 16-byte reduction per crossing).  The per-cell
-// quantities (absorption, source function) are one 32-byte record per cell,
-// one 256-bit load per step.  A second kernel folds the batch's angles into the six
-// per-cell totals in angle order, as calc_GH_tot does angle after angle.
+// B200 design.  The rays of one angle start one per face cell at the same
+// offset and wrap periodically, so they are translations of one path: the
+// same sequence of faces crossed and the same chords, and every cell of the
+// box is crossed by the whole sequence of one layer.  k_art_sweep forms that
+// path once per CTA (in double) and marches 256 rays along it in step; the
+// chord length that the reference sums per cell and angle is then one number
+// per angle (the layer's thickness along the ray), so an angle's term is
+// linear in its crossings and all angles add into one accumulator per cell
+// (vector reductions that stay in L2), closed once at the end.  Angles or
+// boxes without that symmetry (a start face the direction does not enter
+// through, a box that is not the local domain) take the general march
+// (k_art_trace: a float DDA per ray, accumulators per angle, k_art_fold);
+// it also counts the crossings when the caller asks for them.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -120,15 +124,23 @@ __device__ double rec_heiii_b(double t) {
   return 1.3765e-14 * pow(lam, 1.5) / pow(1.0 + pow(lam / 2.740, 0.407), 2.242);
 }
 
+// Index of cell c with y and z exchanged (y fastest): the layout in which the
+// rays of a start face normal to z are neighbours in memory.
+__device__ __forceinline__ uint64_t transposed(uint64_t c, int ny, int nz) {
+  const uint64_t r = c / (uint64_t)nz, iz = c - r * (uint64_t)nz, ix = r / (uint64_t)ny, iy = r - ix * (uint64_t)ny;
+  return (ix * (uint64_t)nz + iz) * (uint64_t)ny + iy;
+}
+
 // ------------------------------------------------------------- per cell
 // Absorption coefficients [cm^-1] and source functions of the three
 // frequencies (calc_rmesh_data.c:33-111, with the reference's float
 // storage), and zeroed totals.  fields: 8 planes of ncell floats: dens,
 // fHI, fHII, fHeI, fHeII, fHeIII, felec, uene (the prev_chem fractions and
-// prev_uene of fluid_mesh).
+// prev_uene of fluid_mesh).  cells_t: a copy with y fastest, or null.
 __global__ void __launch_bounds__(256) k_art_cells(uint64_t n, const float *__restrict__ f, double denstonh,
                                                   double uenetok, float cs_hi, float cs_hei, float cs_heii,
-                                                  ArtCell *__restrict__ cells, float *__restrict__ gh6) {
+                                                  ArtCell *__restrict__ cells, ArtCell *__restrict__ cells_t, int ny,
+                                                  int nz, float *__restrict__ gh6) {
   for (uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < n; c += (uint64_t)gridDim.x * blockDim.x) {
     const float dens = f[c], fhi = f[n + c], fhii = f[2 * n + c], fhei = f[3 * n + c];
     const float fheii = f[4 * n + c], fheiii = f[5 * n + c], felec = f[6 * n + c], uene = f[7 * n + c];
@@ -150,14 +162,16 @@ __global__ void __launch_bounds__(256) k_art_cells(uint64_t n, const float *__re
     const double e1 = (rec_hii_a(t) - rec_hii_b(t)) * ne * nhii * kNuLeV * kThrHI * kEVtoErg / (4.0 * kPi);
     const double e2 = (rec_heii_a(t) - rec_heii_b(t)) * ne * nheii * kNuLeV * kThrHeI * kEVtoErg / (4.0 * kPi);
     const double e3 = (rec_heiii_a(t) - rec_heiii_b(t)) * ne * nheiii * kNuLeV * kThrHeII * kEVtoErg / (4.0 * kPi);
-    cells[c] = ArtCell{a1, a2, a3, (float)(e1 / (double)a1), (float)(e2 / (double)a2), (float)(e3 / (double)a3),
-                       0.f, 0.f};
+    const ArtCell cl{a1, a2, a3, (float)(e1 / (double)a1), (float)(e2 / (double)a2), (float)(e3 / (double)a3),
+                     0.f, 0.f};
+    cells[c] = cl;
+    if (cells_t) cells_t[transposed(c, ny, nz)] = cl;
 #pragma unroll
     for (int s = 0; s < 6; s++) gh6[s * n + c] = 0.f;
   }
 }
 
-// e^-tau and 1 - e^-tau in FP32: the exponential on the SFU, the
+// e^-tau and 1 - e^-tau of the general march in FP32: the exponential on the SFU, the
 // difference by its Taylor series below tau = 1/2 (no cancellation; the
 // truncation after the tau^9 term is below 3e-9 relative there).
 __device__ __forceinline__ void att(float tau, float *et, float *em1) {
@@ -185,9 +199,15 @@ __device__ __forceinline__ void att(float tau, float *et, float *em1) {
 #ifndef ARGOT_ART_MIN_CTAS
 #define ARGOT_ART_MIN_CTAS 6
 #endif
+#ifndef ARGOT_ART_SWEEP_CTAS
+#define ARGOT_ART_SWEEP_CTAS 5
+#endif
 // One thread per ray of angles [a0, a0 + na); acc: na planes of ncell
 // float4 (sum of I (1 - e^-tau) per frequency, chord length).  A ray that
-// exceeds its step bound sets *err and stops.
+// exceeds its step bound sets *err and stops.  kCountOnly: the crossings
+// alone, of angles whose rays k_art_sweep marches (no cells, no accumulators,
+// no error).
+template <bool kCountOnly>
 __global__ void __launch_bounds__(256, ARGOT_ART_MIN_CTAS) k_art_trace(ArtGeom g, const ArtAngle *__restrict__ ang, int a0, int na,
                                                   uint32_t face_max, const ArtCell *__restrict__ cells,
                                                   float4 *__restrict__ acc,
@@ -241,7 +261,7 @@ __global__ void __launch_bounds__(256, ARGOT_ART_MIN_CTAS) k_art_trace(ArtGeom g
       bool inside = ix >= 0 && iy >= 0 && iz >= 0 && ix < g.nx && iy < g.ny && iz < g.nz;
       while (inside) {
         if (steps >= cap) {
-          atomicExch(err, 1);
+          if (!kCountOnly) atomicExch(err, 1);
           break;
         }
         steps++;
@@ -261,6 +281,7 @@ __global__ void __launch_bounds__(256, ARGOT_ART_MIN_CTAS) k_art_trace(ArtGeom g
         if (rdx == rmin) ix += xn;
         if (rdy == rmin) iy += yn;
         if (rdz == rmin) iz += zn;
+        if (!kCountOnly) {
         rmin = __double2float_rn(__dmul_rn((double)rmin, g.lunit));
         // intensities (calc_intensity, ray_tracing.c:71-157)
         const ArtCell cl = load_cell(cells + pos);
@@ -277,6 +298,7 @@ __global__ void __launch_bounds__(256, ARGOT_ART_MIN_CTAS) k_art_trace(ArtGeom g
         i3 = fmaf(i3, et, cl.s3 * em);
         add.w = rmin;
         atomicAdd(accA + pos, add);
+        }
         // leaving the box: stop at the far face, wrap through the side faces
         // with the intensity reset (ray_tracing.c:276-372, one rank)
         if (ix >= g.nx || iy >= g.ny || iz >= g.nz || ix < 0 || iy < 0 || iz < 0) {
@@ -353,12 +375,252 @@ __global__ void __launch_bounds__(256) k_art_fold(uint64_t n, int na, const floa
   }
 }
 
-// rates6 += totals / N_ANG (calc_GH_sum, calc_GH_tot.c:232-247)
-__global__ void __launch_bounds__(256) k_art_add(uint64_t n, const float *__restrict__ gh6, float r_nang,
-                                                float *__restrict__ rates6) {
+// ---------------------------------------------------------------- sweep
+// The path shared by the rays of one angle: faces of the start axis at path
+// lengths (j + 1) T, of a side axis at (f + k) T, f the distance of the start
+// point from its first face in cells, T the face spacing along the ray.
+struct ArtAxis {
+  double T, f;
+  int n;  // faces before the end of the path
+  __device__ __forceinline__ double at(int k) const { return (f + (double)k) * T; }
+  // faces with path length below s (or at s, kUpTo)
+  template <bool kUpTo>
+  __device__ __forceinline__ int count(double s) const {
+    int k = (int)fmin(fmax(s / T - f, 0.0), 1.0e9);
+    while (k > 0 && !(kUpTo ? at(k - 1) <= s : at(k - 1) < s)) k--;
+    while (kUpTo ? at(k) <= s : at(k) < s) k++;
+    return min(k, n);
+  }
+};
+constexpr int kArtMaxSteps = 3072;  // steps of a path held in shared memory
+constexpr int kArtThreads = 256;
+constexpr uint64_t kArtWaves = 4;
+
+// e^-tau and 1 - e^-tau from y = tau log2(e) / 2: below tau = 1, 1 - e^-tau =
+// tau e^(-tau/2) sinh(tau/2)/(tau/2) with the polynomial of the FP32 rates
+// (argot_b200/fits.py, in (2 y)^2; no cancellation, within 1.5e-7), above, the
+// difference.
+__device__ __forceinline__ void att_y(float y, float *et, float *em1) {
+  constexpr float k = 1.38629436f;  // tau = 2 ln2 y
+  float h;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(h) : "f"(-y));
+  const float v = y * y, e = h * h;
+  const float p = fmaf(v, fmaf(v, fmaf(v, k * 64.f * 3.4621803e-07f, k * 16.f * 0.000120223514f), k * 4.f * 0.0200188775f), k);
+  *et = e;
+  *em1 = y < 0.72134752f ? y * (h * p) : 1.f - e;
+}
+
+// What bounds the sweep at 128^3 cells / 768 directions (12.1 ms a pass; the
+// general march with its per-angle accumulators, 64 angles at a time, took
+// 33.4 ms and moved 52 GB of accumulators through DRAM): issue, 81% of the
+// cycles, then the reductions on the way to L2 (68% of that path; one per
+// crossing: 81%, 12.5 ms).  Without the copy with y fastest, the rays of the
+// faces normal to z read and reduce one line per lane: 17.0 ms.  5 CTAs per
+// SM (48 registers); 4: 12.3 ms, 6: 12.4 ms.
+//
+// One CTA: 256 rays of one angle (blockIdx.y), marched together along the
+// angle's path.  A step's axis is the same for all rays, so a ray keeps its
+// cell index and, per side axis, the steps to its wrap.  Rays are taken in
+// tiles of 8 rows of 32 cells of the start face, so that a side step finds
+// the cells its neighbours just read in L1.  acc[c] += (I (1 - e^-tau)) d / L
+// per frequency, L the layer's path length and d the smallest cell side (a
+// factor of order one, so that the sums keep the intensities' range).  The
+// next step's cell is loaded before this step's arithmetic.  cells_t, acc_t:
+// the layout with y fastest for the start faces normal to z, whose rays would
+// otherwise lie a row apart (null: none).
+__global__ void __launch_bounds__(kArtThreads, ARGOT_ART_SWEEP_CTAS)
+    k_art_sweep(ArtGeom g, const ArtAngle *__restrict__ ang, int a0, const ArtCell *__restrict__ cells,
+                float4 *__restrict__ acc, const ArtCell *__restrict__ cells_t, float4 *__restrict__ acc_t) {
+  // per step: chord [cm] times log2(e) / 2, the cell index's change, 1 for a
+  // step along p, 1 for a step along q
+  extern __shared__ float4 s_path[];
+  const ArtAngle A = ang[a0 + blockIdx.y];
+  const int nn[3] = {g.nx, g.ny, g.nz};
+  const double o[3] = {A.ox, A.oy, A.oz}, dd[3] = {g.dx, g.dy, g.dz};
+  const double off[3] = {0.521212345, 0.508512345, 0.468287655};
+  const int ax = A.base < 2 ? 2 : A.base < 4 ? 0 : 1;  // start axis
+  const int p = ax == 0 ? 1 : 0, q = ax == 2 ? 1 : 2;  // side axes, q the faster one in memory
+  const ArtAxis B{dd[ax] / fabs(o[ax]), 1.0, nn[ax]};
+  const double end = B.at(B.n - 1);
+  ArtAxis P{dd[p] / fabs(o[p]), o[p] > 0.0 ? 1.0 - off[p] : off[p], 1 << 30};
+  ArtAxis Q{dd[q] / fabs(o[q]), o[q] > 0.0 ? 1.0 - off[q] : off[q], 1 << 30};
+  P.n = P.count<false>(end);
+  Q.n = Q.count<false>(end);
+  const int nstep = B.n + P.n + Q.n;
+  const bool tr = ax == 2 && cells_t;
+  if (tr) {
+    cells = cells_t;
+    acc = acc_t;
+  }
+  const int64_t st[3] = {(int64_t)g.ny * g.nz, tr ? 1 : (int64_t)g.nz, tr ? (int64_t)g.ny : 1};
+  // index changes of a step, modulo 2^32 as the index itself
+  const uint32_t db = (uint32_t)(o[ax] > 0.0 ? st[ax] : -st[ax]);
+  const uint32_t dp = (uint32_t)(o[p] > 0.0 ? st[p] : -st[p]), dq = (uint32_t)(o[q] > 0.0 ? st[q] : -st[q]);
+  // a face's rank in the path: the faces of each axis before it (of equal
+  // ones the start axis's first, then p's), its chord from the latest of those
+  for (int i = threadIdx.x; i < nstep; i += kArtThreads) {
+    int t = 0, kb = i, kp, kq;
+    double s;
+    if (i < B.n) {
+      s = B.at(kb);
+      kp = P.count<false>(s);
+      kq = Q.count<false>(s);
+    } else if (i < B.n + P.n) {
+      t = 1;
+      kp = i - B.n;
+      s = P.at(kp);
+      kb = B.count<true>(s);
+      kq = Q.count<false>(s);
+    } else {
+      t = 2;
+      kq = i - B.n - P.n;
+      s = Q.at(kq);
+      kb = B.count<true>(s);
+      kp = P.count<true>(s);
+    }
+    double s0 = 0.0;
+    if (kb > 0) s0 = fmax(s0, B.at(kb - 1));
+    if (kp > 0) s0 = fmax(s0, P.at(kp - 1));
+    if (kq > 0) s0 = fmax(s0, Q.at(kq - 1));
+    s_path[kb + kp + kq] =
+        make_float4((float)((s - s0) * g.lunit * 0.72134752044448170), __uint_as_float(t == 0 ? db : t == 1 ? dp : dq),
+                    __int_as_float(t == 1), __int_as_float(t == 2));
+  }
+  __syncthreads();
+  // this thread's ray: cell (ip, iq) of the start face
+  const uint32_t np = (uint32_t)nn[p], nq = (uint32_t)nn[q];
+  const uint32_t r = blockIdx.x * kArtThreads + threadIdx.x;
+  const unsigned mask = __ballot_sync(0xffffffffu, r < np * nq);
+  if (r >= np * nq) return;
+  const uint32_t strip = r / (8u * nq), rows = min(8u, np - 8u * strip), in = r - strip * 8u * nq;
+  const uint32_t chunk = in / (32u * rows), cols = min(32u, nq - 32u * chunk), at = in - chunk * 32u * rows;
+  const uint32_t ip = 8u * strip + at / cols, iq = 32u * chunk + at % cols;
+  uint32_t pos = (uint32_t)(ip * st[p] + iq * st[q] + (o[ax] > 0.0 ? 0 : (nn[ax] - 1) * st[ax]));
+  int wp = o[p] > 0.0 ? (int)(np - ip) : (int)ip + 1, wq = o[q] > 0.0 ? (int)(nq - iq) : (int)iq + 1;
+  const float il = (float)(fmin(dd[0], fmin(dd[1], dd[2])) / B.T);  // d / L
+  // the lane whose ray runs one cell ahead along q, the same row's next cell in
+  // that direction (periodically: the rays keep their distance), and whether
+  // there is a lane one cell behind
+  const int lane = threadIdx.x & 31, dir = o[q] > 0.0 ? 1 : -1;
+  const bool next_in_row = at % cols + 1 < cols, prev_in_row = at % cols > 0;
+  const bool has_ahead = dir > 0 ? next_in_row && lane < 31 && (mask >> (lane + 1) & 1u) : prev_in_row && lane > 0;
+  const bool has_behind = dir > 0 ? prev_in_row && lane > 0 : next_in_row && lane < 31 && (mask >> (lane + 1) & 1u);
+  const int ahead = has_ahead ? lane + dir : lane;
+  float m1 = 0.f, m2 = 0.f, m3 = 0.f;  // sums of the current cell not yet added to acc
+  float i1 = 0.f, i2 = 0.f, i3 = 0.f;  // intensities
+  ArtCell cl = load_cell(cells + pos);
+#pragma unroll 2
+  for (int k = 0; k < nstep; k++) {
+    const float4 step = s_path[k];
+    const bool along_q = __any_sync(mask, __float_as_int(step.w));  // (uniform, known to the compiler as such)
+    uint32_t nxt = pos + __float_as_uint(step.y);
+    bool wrapped = false;
+    wp -= __float_as_int(step.z);
+    wq -= __float_as_int(step.w);
+    if (wp == 0 || wq == 0) {
+      wrapped = true;
+      if (wp == 0) {
+        nxt -= np * dp;
+        wp = (int)np;
+      } else {
+        nxt -= nq * dq;
+        wq = (int)nq;
+      }
+    }
+    // (past the last step the ray has left through the far face)
+    const ArtCell cn = load_cell(cells + (k + 1 < nstep ? nxt : pos));
+    const float c = step.x;
+    if (c > 0.f) {
+      float et, em;
+      att_y(cl.a1 * c, &et, &em);
+      m1 = fmaf(i1, em, m1);
+      i1 = fmaf(i1, et, cl.s1 * em);
+      att_y(cl.a2 * c, &et, &em);
+      m2 = fmaf(i2, em, m2);
+      i2 = fmaf(i2, et, cl.s2 * em);
+      att_y(cl.a3 * c, &et, &em);
+      m3 = fmaf(i3, em, m3);
+      i3 = fmaf(i3, et, cl.s3 * em);
+    }
+    // leaving along q, the ray enters the cell of the lane ahead, whose sums
+    // it takes over; else, and where no lane follows, the sums go to memory
+    if (along_q) {
+      if (!has_behind) atomicAdd(acc + pos, make_float4(m1 * il, m2 * il, m3 * il, 0.f));
+      m1 = __shfl_sync(mask, m1, ahead);
+      m2 = __shfl_sync(mask, m2, ahead);
+      m3 = __shfl_sync(mask, m3, ahead);
+      if (!has_ahead) m1 = m2 = m3 = 0.f;
+    } else {
+      atomicAdd(acc + pos, make_float4(m1 * il, m2 * il, m3 * il, 0.f));
+      m1 = m2 = m3 = 0.f;
+    }
+    if (wrapped) i1 = i2 = i3 = 0.f;
+    pos = nxt;
+    cl = cn;
+  }
+}
+
+// A group's sums added to the running totals (compensated: planes 0..2 sums,
+// 3..5 compensations) and the accumulators cleared for the next group.
+__global__ void __launch_bounds__(256) k_art_gather(uint64_t n, int ny, int nz, float4 *__restrict__ acc,
+                                                   float4 *__restrict__ acc_t, float *__restrict__ tot6) {
   for (uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < n; c += (uint64_t)gridDim.x * blockDim.x) {
+    float4 v = acc[c];
+    acc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (acc_t) {
+      float4 *w = acc_t + transposed(c, ny, nz);
+      v = make_float4(v.x + w->x, v.y + w->y, v.z + w->z, 0.f);
+      *w = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const float add[3] = {v.x, v.y, v.z};
 #pragma unroll
-    for (int s = 0; s < 6; s++) rates6[s * n + c] = __fadd_rn(rates6[s * n + c], __fmul_rn(gh6[s * n + c], r_nang));
+    for (int q = 0; q < 3; q++) {
+      const float y = add[q] - tot6[(3 + q) * n + c], t0 = tot6[q * n + c], t = t0 + y;
+      tot6[(3 + q) * n + c] = (t - t0) - y;
+      tot6[q * n + c] = t;
+    }
+  }
+}
+
+// The six rates of a cell from the swept angles' sums m_i = sum over angles
+// of (sum of I (1 - e^-tau)) d / L, id = 1 / d [cm^-1] and the number of those angles
+// (calc_GH_tot.c:178-247), plus the general march's totals gh6, over all
+// angles.  tot6: gh6 (kGeneral) or the earlier groups' totals.
+template <bool kGeneral>
+__global__ void __launch_bounds__(256) k_art_close(uint64_t n, int ny, int nz, const float4 *__restrict__ acc,
+                                                  const float4 *__restrict__ acc_t, const float *__restrict__ tot6,
+                                                  const ArtCell *__restrict__ cells,
+                                                  ArtStep st, float nswept, float id, float r_nang,
+                                                  float *__restrict__ rates6) {
+  for (uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < n; c += (uint64_t)gridDim.x * blockDim.x) {
+    const ArtCell cl = load_cell(cells + c);
+    const float4 v = acc[c];
+    float m1 = v.x, m2 = v.y, m3 = v.z;
+    if (acc_t) {
+      const float4 w = acc_t[transposed(c, ny, nz)];
+      m1 += w.x;
+      m2 += w.y;
+      m3 += w.z;
+    }
+    if (!kGeneral) {
+      m1 = tot6[c] + (m1 - tot6[3 * n + c]);
+      m2 = tot6[n + c] + (m2 - tot6[4 * n + c]);
+      m3 = tot6[2 * n + c] + (m3 - tot6[5 * n + c]);
+    }
+    const float j1 = fmaf(nswept, cl.s1, m1 / cl.a1 * id), j2 = fmaf(nswept, cl.s2, m2 / cl.a2 * id),
+                j3 = fmaf(nswept, cl.s3, m3 / cl.a3 * id);
+    float gh[6];
+    gh[0] = fmaf(j3, (float)kRintJHI3, fmaf(j2, (float)kRintJHI2, j1)) * st.f[0];
+    gh[3] = fmaf(j3, (float)kRintHHI3, fmaf(j2, (float)kRintHHI2, j1)) * st.f[1];
+    gh[1] = fmaf(j3, (float)kRintJHeI3, j2) * st.f[2];
+    gh[4] = fmaf(j3, (float)kRintHHeI3, j2) * st.f[3];
+    gh[2] = j3 * st.f[4];
+    gh[5] = j3 * st.f[5];
+#pragma unroll
+    for (int s = 0; s < 6; s++) {
+      if (kGeneral) gh[s] += tot6[s * n + c];
+      rates6[s * n + c] = __fadd_rn(rates6[s * n + c], __fmul_rn(gh[s], r_nang));
+    }
   }
 }
 
@@ -498,12 +760,45 @@ struct argot_b200_art {
   int device;
   int nang;
   argot::ArtAngle *dev_ang;
+  std::vector<argot::ArtAngle> ang;  // the same on the host
   argot::ArtStep step;
 };
 
 using namespace argot;
 
 namespace {
+
+// The box is the local domain, to a thousandth of a cell, on every axis.
+bool art_box_is_local(const ArtGeom &g) {
+  const double lo[3] = {g.xmin, g.ymin, g.zmin}, hi[3] = {g.xmax, g.ymax, g.zmax};
+  const double ll[3] = {g.xminl, g.yminl, g.zminl}, hl[3] = {g.xmaxl, g.ymaxl, g.zmaxl};
+  const double d[3] = {g.dx, g.dy, g.dz};
+  const int n[3] = {g.nx, g.ny, g.nz};
+  for (int k = 0; k < 3; k++) {
+    const double tol = 1e-3 * d[k];
+    if (!(std::fabs(lo[k] - ll[k]) <= tol && std::fabs(hi[k] - hl[k]) <= tol &&
+          std::fabs(ll[k] + n[k] * d[k] - hl[k]) <= tol))
+      return false;
+  }
+  return std::isfinite(g.lunit) && g.lunit > 0.0;
+}
+
+// Steps of the path that the rays of one angle share, 0 when they do not
+// share one: the direction must enter through the start face.  (An upper
+// bound: a side face that falls on the path's end may be counted.)
+int art_path_steps(const ArtGeom &g, const ArtAngle &A) {
+  const double o[3] = {A.ox, A.oy, A.oz}, d[3] = {g.dx, g.dy, g.dz};
+  const int n[3] = {g.nx, g.ny, g.nz}, ax = A.base < 2 ? 2 : A.base < 4 ? 0 : 1;
+  for (double v : o)
+    if (!std::isfinite(v) || v == 0.0) return 0;
+  if ((o[ax] > 0.0) != (A.base % 2 == 0)) return 0;
+  const double end = n[ax] * d[ax] / std::fabs(o[ax]);
+  double steps = n[ax];
+  for (int k = 0; k < 3; k++)
+    if (k != ax) steps += std::floor(end * std::fabs(o[k]) / d[k]) + 2.0;
+  if (!(steps <= kArtMaxSteps) || steps >= 8.0 * ((double)g.nx + g.ny + g.nz) + 16.0) return 0;
+  return (int)steps;
+}
 
 int art_run(const argot_b200_art *a, const ArtGeom &g, double denstonh, double uenetok, const float *fields8,
             float *rates6, void *work, int apass, unsigned long long *crossings, int *err, cudaStream_t st) {
@@ -514,22 +809,94 @@ int art_run(const argot_b200_art *a, const ArtGeom &g, double denstonh, double u
   const int blocks = art_blocks(n);
   const float cs1 = (float)sigma_hi(kThrHI + 1.0e-7), cs2 = (float)sigma_hei(kThrHeI + 1.0e-7);
   const float cs3 = (float)sigma_heii(kThrHeII + 1.0e-7);
-  k_art_cells<<<blocks, 256, 0, st>>>(n, fields8, denstonh, uenetok, cs1, cs2, cs3, cells, gh6);
-  ARGOT_CUDA_TRY(cudaGetLastError());
   const uint32_t face_max = (uint32_t)std::max<uint64_t>(
       (uint64_t)g.nx * g.ny, std::max<uint64_t>((uint64_t)g.ny * g.nz, (uint64_t)g.nz * g.nx));
-  for (int a0 = 0; a0 < a->nang; a0 += apass) {
-    const int na = std::min(apass, a->nang - a0);
-    ARGOT_CUDA_TRY(cudaMemsetAsync(acc, 0, sizeof(float4) * n * (uint64_t)na, st));
-    const uint64_t threads = (uint64_t)na * face_max;
-    k_art_trace<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(g, a->dev_ang, a0, na, face_max, cells, acc,
-                                                                    crossings, err);
-    ARGOT_CUDA_TRY(cudaGetLastError());
-    k_art_fold<<<blocks, 256, 0, st>>>(n, na, acc, cells, a->step, gh6);
-    ARGOT_CUDA_TRY(cudaGetLastError());
+  // the angles whose rays share a path are swept, the others marched one ray
+  // at a time; both in runs of consecutive angles
+  const bool local = art_box_is_local(g);
+  auto steps = [&](int i) { return local ? art_path_steps(g, a->ang[(size_t)i]) : 0; };
+  int nswept = 0, most = 0;
+  for (int i = 0; i < a->nang; i++) {
+    const int k = steps(i);
+    nswept += k > 0;
+    most = std::max(most, k);
+  }
+  auto run_end = [&](int i) {
+    const bool s = steps(i) > 0;
+    int j = i + 1;
+    while (j < a->nang && (steps(j) > 0) == s) j++;
+    return j;
+  };
+  const bool general = nswept < a->nang;
+  // four planes or more, all free of the general march, also hold the copies
+  // with y fastest (the cells' copy first: its records are 32-byte aligned)
+  ArtCell *cells_t = nullptr;
+  float4 *acc_t = nullptr;
+  if (!general && apass >= 4) {
+    cells_t = cells + n;
+    acc = (float4 *)(cells_t + n);
+    acc_t = acc + n;
+  }
+  k_art_cells<<<blocks, 256, 0, st>>>(n, fields8, denstonh, uenetok, cs1, cs2, cs3, cells, cells_t, g.ny, g.nz, gh6);
+  ARGOT_CUDA_TRY(cudaGetLastError());
+  for (int i = 0; i < a->nang; i = run_end(i)) {
+    const int j = run_end(i);
+    if (steps(i) > 0) {
+      for (int a0 = i; crossings && a0 < j; a0 += apass) {
+        const int na = std::min(apass, j - a0);
+        const uint64_t threads = (uint64_t)na * face_max;
+        k_art_trace<true><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(g, a->dev_ang, a0, na, face_max, cells,
+                                                                              acc, crossings, err);
+        ARGOT_CUDA_TRY(cudaGetLastError());
+      }
+      continue;
+    }
+    for (int a0 = i; a0 < j; a0 += apass) {
+      const int na = std::min(apass, j - a0);
+      ARGOT_CUDA_TRY(cudaMemsetAsync(acc, 0, sizeof(float4) * n * (uint64_t)na, st));
+      const uint64_t threads = (uint64_t)na * face_max;
+      k_art_trace<false><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(g, a->dev_ang, a0, na, face_max, cells,
+                                                                             acc, crossings, err);
+      ARGOT_CUDA_TRY(cudaGetLastError());
+      k_art_fold<<<blocks, 256, 0, st>>>(n, na, acc, cells, a->step, gh6);
+      ARGOT_CUDA_TRY(cudaGetLastError());
+    }
+  }
+  ARGOT_CUDA_TRY(cudaMemsetAsync(acc, 0, sizeof(float4) * n, st));
+  if (acc_t) ARGOT_CUDA_TRY(cudaMemsetAsync(acc_t, 0, sizeof(float4) * n, st));
+  // groups of angles per launch: enough CTAs for kArtWaves fills of the GPU
+  // and at least 128 angles; between groups the sums (of about 2 terms per
+  // angle) go into compensated totals
+  const uint32_t tiles = (face_max + kArtThreads - 1) / kArtThreads;
+  const int group = (int)std::max<uint64_t>(128, (kArtWaves * 148 * ARGOT_ART_SWEEP_CTAS + tiles - 1) / tiles);
+  int in_group = 0;
+  for (int i = 0, left = nswept; left > 0; i = run_end(i)) {
+    if (steps(i) == 0) continue;
+    const int j = run_end(i);
+    for (int a0 = i; a0 < j;) {
+      if (in_group >= group && !general) {
+        k_art_gather<<<blocks, 256, 0, st>>>(n, g.ny, g.nz, acc, acc_t, gh6);
+        ARGOT_CUDA_TRY(cudaGetLastError());
+        in_group = 0;
+      }
+      const int na = std::min(std::min(j - a0, 32768), general ? 32768 : group - in_group);
+      k_art_sweep<<<dim3(tiles, (unsigned)na), kArtThreads, sizeof(float4) * (size_t)most, st>>>(g, a->dev_ang, a0,
+                                                                                                  cells, acc, cells_t,
+                                                                                                  acc_t);
+      ARGOT_CUDA_TRY(cudaGetLastError());
+      in_group += na;
+      a0 += na;
+      left -= na;
+    }
   }
   const float r_nang = (float)(1.0e0 / a->nang);
-  k_art_add<<<blocks, 256, 0, st>>>(n, gh6, r_nang, rates6);
+  const float id = (float)(1.0 / ((double)std::min(g.dx, std::min(g.dy, g.dz)) * g.lunit));
+  if (general)
+    k_art_close<true><<<blocks, 256, 0, st>>>(n, g.ny, g.nz, acc, acc_t, gh6, cells, a->step, (float)nswept, id, r_nang,
+                                             rates6);
+  else
+    k_art_close<false><<<blocks, 256, 0, st>>>(n, g.ny, g.nz, acc, acc_t, gh6, cells, a->step, (float)nswept, id, r_nang,
+                                             rates6);
   ARGOT_CUDA_TRY(cudaGetLastError());
   return 0;
 }
@@ -718,6 +1085,7 @@ int argot_b200_art_create(const float *dir3, const int *base_corner2, int nang, 
   argot_b200_art *a = new (std::nothrow) argot_b200_art();
   if (!a) { set_status(ARGOT_B200_ENOMEM); return ARGOT_B200_ENOMEM; }
   a->nang = nang;
+  a->dev_ang = nullptr;
   for (int s = 0; s < 6; s++) a->step.f[s] = step6[s];
   cudaError_t e = cudaGetDevice(&a->device);
   if (e == cudaSuccess) e = cudaMalloc(&a->dev_ang, sizeof(ArtAngle) * (size_t)nang);
@@ -728,6 +1096,7 @@ int argot_b200_art_create(const float *dir3, const int *base_corner2, int nang, 
     delete a;
     return status_from_cuda(e);
   }
+  a->ang.swap(h);
   *out = a;
   set_status(0);
   return 0;
