@@ -150,3 +150,38 @@ def test_dropin_smooth_photoion_rate(cuda_ok, edge, isolated):
             assert np.array_equal(got2["prev_chem"][n], twice[k]), n
     finally:
         lib.argot_b200_set_dropin_smooth_faces(1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("isolated", [True, False])
+@pytest.mark.parametrize("n", [(1, 1, 1), (2, 3, 33), (7, 1, 64), (25, 6, 31), (49, 4, 97), (30, 5, 32), (3, 2, 1)])
+def test_device_smoothing_ragged(cuda_ok, n, isolated):
+    """Meshes whose axes are no multiple of the kernel's rows, segments and
+    32 cells along z, with zeros, subnormals and infinities among the rates:
+    the same bits as the restatement."""
+    import torch
+    from argot_b200 import _lib as L
+    import ctypes as C
+    rng = np.random.default_rng(sum(n))
+    x = (10.0 ** rng.normal(-12, 3, (6,) + n)).astype(np.float32)
+    x[0, rng.random(n) < 0.2] = 0.0
+    x[1] *= np.float32(1e-30)
+    x[2].flat[n[0] * n[1] * n[2] // 2] = np.inf
+    want = np.empty_like(x)
+    for s in range(6):
+        p = np.pad(x[s], 1, mode="edge" if isolated else "wrap")
+        terms = [p[1 + a:1 + a + n[0], 1 + b:1 + b + n[1], 1 + c:1 + c + n[2]]
+                 for a in (-1, 0, 1) for b in (-1, 0, 1) for c in (-1, 0, 1)]
+        acc = terms[0]
+        for t in terms[1:13]:
+            acc = acc + t
+        d = acc.astype(np.float64) + SM.CENTRAL_WEIGHT * terms[13].astype(np.float64)
+        for t in terms[14:]:
+            d = d + t.astype(np.float64)
+        want[s] = (SM.NORMAL * d).astype(np.float32)
+    g = L.Grid(*n, 0, 0, 0, 0.0, 0.0, 0.0, *map(float, n), 0.0, 0.0, 0.0, 1.0, 1.0, 1.0, 1.0, 1.0)
+    xin = torch.from_numpy(x.ravel().copy()).cuda()
+    out = torch.full_like(xin, -1.0)
+    L.check(L.load().argot_b200_smooth_rates(C.byref(g), xin.data_ptr(), out.data_ptr(), int(isolated),
+                                             torch.cuda.current_stream().cuda_stream), "smooth_rates")
+    assert np.array_equal(out.cpu().numpy().reshape(want.shape), want)
