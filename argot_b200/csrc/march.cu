@@ -148,9 +148,12 @@ __global__ void __launch_bounds__(256) k_walk(GridDev g, const DevNode *__restri
 // 16 warps 0.629 s).  What bounds it now: the L1 data pipe (77% of its peak,
 // one line per cycle for each quarter warp of a 16-byte gather), the ALU
 // (68%) and issue (71%) together.
-// Launch shape: 64 warps per SM (32 registers) in CTAs of 32 warps; a range
-// of blocks that would leave SMs empty that way (fewer than kWideBlocks)
-// takes CTAs of 8 warps.  What lives across a ray's walk is kept out of
+// Launch shape: 64 warps per SM (32 registers) in CTAs of 32 warps.  A range
+// of few blocks is cut finer: each block's chunks of 32 rays into segments,
+// one warp each, until there are kMarchItems items per warp slot (32^3 cells
+// / 8 sources: 78 -> 41 us, 64^3 / 16: 0.49 -> 0.45 ms; more items per slot
+// on larger meshes: no change), in CTAs of 8 warps where 32 would leave SMs
+// empty.  What lives across a ray's walk is kept out of
 // registers: the Kahan columns in per-thread shared-memory slots, the
 // block's state (item, ray count, packed coordinates, first ray; the same
 // for the warp's lanes) in per-warp shared memory, read back after each ray.
@@ -158,7 +161,7 @@ __global__ void __launch_bounds__(256) k_walk(GridDev g, const DevNode *__restri
 // bounding box), so rays start at their emitter and the launch contains no
 // call.
 constexpr int kMarchWide = 1024, kMarchNarrow = 256;
-constexpr uint64_t kWideBlocks = 148 * 64;
+constexpr uint64_t kMarchItems = 2;
 
 // One level of a tiled enumeration of nx * ny * nz blocks (tiles of tx * ty *
 // tz, those at the high ends clipped; tiles in (x, y, z) order with z
@@ -209,8 +212,9 @@ template <int kPrec, bool kInside, int kThreads>
 __global__ void __launch_bounds__(kThreads, 2048 / kThreads) k_march_rays(GridDev g, const float4 *__restrict__ cells,
                                                     const float4 *__restrict__ emit_pos, uint32_t b0,
                                                     uint32_t b1, const uint64_t *__restrict__ blk_off,
-                                                    uint64_t base, const uint32_t *__restrict__ rays,
-                                                    uint64_t nray, float *__restrict__ tau,
+                                                    uint32_t nseg, uint64_t base,
+                                                    const uint32_t *__restrict__ rays, uint64_t nray,
+                                                    float *__restrict__ tau,
                                                     unsigned long long *__restrict__ crossings,
                                                     int *__restrict__ err) {
   const int lane = threadIdx.x & 31;
@@ -223,10 +227,24 @@ __global__ void __launch_bounds__(kThreads, 2048 / kThreads) k_march_rays(GridDe
   __shared__ uint32_t wstate[kThreads / 32][5];
   volatile uint32_t *ws = wstate[threadIdx.x >> 5];
   bool bad = false;
-  for (uint32_t it = b0 + warp; it < b1; it += nwarp) {
-    const uint32_t b = block_of_item((uint32_t)g.nby, (uint32_t)g.nbz, it, b0, b1);
+  // item it: segment (it / W) % nseg of the block whose rank in the range is
+  // it / (W nseg) * W + it % W, W the warps of a CTA, which so hold the same
+  // segment of neighbouring blocks
+  constexpr uint32_t W = kThreads / 32;
+  const uint32_t nitem = (b1 - b0 + W - 1) / W * W * nseg;
+  for (uint32_t it = warp; it < nitem; it += nwarp) {
+    const uint32_t cw = it / W, grp = cw / nseg, sg = cw - grp * nseg;
+    const uint32_t rank = grp * W + (it - cw * W);
+    if (rank >= b1 - b0) continue;
+    const uint32_t b = block_of_item((uint32_t)g.nby, (uint32_t)g.nbz, b0 + rank, b0, b1);
     uint64_t r0, r1;
     if (!block_rays(blk_off, b, base, nray, &r0, &r1)) { bad = true; continue; }
+    if (nseg > 1) {  // the segment's share of the block's chunks of 32 rays
+      const uint32_t nch = (uint32_t)((r1 - r0 + 31) >> 5);
+      const uint32_t c0 = (uint32_t)((uint64_t)nch * sg / nseg), c1 = (uint32_t)((uint64_t)nch * (sg + 1) / nseg);
+      r1 = min(r1, r0 + (uint64_t)c1 * 32);
+      r0 += (uint64_t)c0 * 32;
+    }
     // the block's coordinates in blocks (the host checks nbx < 4096 and
     // nby, nbz < 1024)
     const uint32_t nyz = (uint32_t)g.nby * (uint32_t)g.nbz;
@@ -483,16 +501,23 @@ int argot_b200_march_rays(const argot_b200_grid *gp, const void *packed, const a
   int *err = err_flag(dev);
   if (!err) { set_status(ARGOT_B200_ENOMEM); return ARGOT_B200_ENOMEM; }
   cudaStream_t st = (cudaStream_t)stream;
-  const bool wide = b1 - b0 >= kWideBlocks;
+  // segments per block: enough items for kMarchItems per warp slot, at most
+  // one per chunk of 32 rays of an average block
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const uint64_t nblk = b1 - b0, slots = 64ull * sms;
+  uint64_t nseg = std::min((kMarchItems * slots + nblk - 1) / nblk, (nray / nblk + 31) / 32);
+  nseg = std::max<uint64_t>(1, std::min<uint64_t>(nseg, 64));
+  const bool wide = nblk * nseg >= slots;
   const int threads = wide ? kMarchWide : kMarchNarrow;
-  const int blocks = grid_blocks_for((b1 - b0) * 32, threads);
+  const int blocks = grid_blocks_for(nblk * nseg * 32, threads);
   const bool inside = t->emit_lo[0] >= gp->xmin && t->emit_lo[1] >= gp->ymin && t->emit_lo[2] >= gp->zmin &&
                       t->emit_hi[0] <= gp->xmax && t->emit_hi[1] <= gp->ymax && t->emit_hi[2] <= gp->zmax;
   const float4 *cells = (const float4 *)packed;
 #define ARGOT_MARCH_LAUNCH(P, I)                                                            \
   (wide ? k_march_rays<P, I, kMarchWide> : k_march_rays<P, I, kMarchNarrow>)                \
       <<<blocks, threads, 0, st>>>(g, cells, t->emit_pos, (uint32_t)b0, (uint32_t)b1,       \
-                                   blk_off, base, rays, nray, tau, crossings, err)
+                                   blk_off, (uint32_t)nseg, base, rays, nray, tau, crossings, err)
   if (prec == ARGOT_B200_PRECISION_REFERENCE) {
     if (inside) ARGOT_MARCH_LAUNCH(ARGOT_B200_PRECISION_REFERENCE, true);
     else ARGOT_MARCH_LAUNCH(ARGOT_B200_PRECISION_REFERENCE, false);

@@ -524,6 +524,50 @@ __device__ __forceinline__ void add_chunk_in_order(Acc &acc, int lane, int t, co
   }
 }
 
+// Phases A and B of a chunk of 32 rays [rc, min(rc + 32, r1)) of a block whose
+// first cell is (bix, biy, biz): S.c.out holds the rays' rates; returns the
+// target lane of ray rc + lane (-1: none).  Ends with the warp synchronised.
+template <bool kServed>
+__device__ __forceinline__ int rate_chunk(const GridDev &g, const float4 *__restrict__ raw,
+                                          const float4 *__restrict__ emit_pos, const float *__restrict__ specn,
+                                          const double *__restrict__ total, const RateLane &tab, int bix, int biy,
+                                          int biz, uint64_t rc, uint64_t r1, const uint32_t *__restrict__ rays,
+                                          uint64_t nray, const float *__restrict__ tau, RateWarpSmem &S, int lane,
+                                          const float *__restrict__ pred) {
+  const uint64_t r = rc + lane;
+  int t = -1;
+  bool quad = false;
+  if (r < r1) {
+    const uint32_t w = __ldg(rays + r);
+    const uint32_t e = w >> 5;
+    t = (int)(w & 31u);
+    if (kServed && __ldg(pred + 6 * nray + r) != 0.f) {
+#pragma unroll
+      for (int s = 0; s < 6; s++) S.c.out[lane][s] = __ldg(pred + s * nray + r);
+    } else {
+      quad = true;
+      const int lx = bix + (t >> 4), ly = biy + ((t >> 2) & 3), lz = biz + (t & 3);
+      const float4 ep = __ldg(emit_pos + e);
+      const float4 rw = __ldg(raw + cell_index(g, lx, ly, lz));
+      const RayParams p = ray_params_f32(g, g.ix0 + lx, g.iy0 + ly, g.iz0 + lz, ep.x, ep.y, ep.z, __ldg(tau + r),
+                                         __ldg(tau + nray + r), __ldg(tau + 2 * nray + r), rw, __ldg(total + e));
+      S.c.rec[lane] = ray_rec(p, (int)e);
+#pragma unroll
+      for (int s = 0; s < 3; s++) S.c.p[lane][s] = p.P[s];
+    }
+  }
+  int nq = (int)min((uint64_t)32, r1 - rc);
+  if (kServed) {
+    const unsigned m = __ballot_sync(0xffffffffu, quad);
+    if (quad) S.q[__popc(m & ((1u << lane) - 1u))] = lane;
+    nq = __popc(m);
+  }
+  __syncwarp();
+  chunk_rates(S.c, tab, specn, kServed ? S.q : nullptr, nq, lane);
+  __syncwarp();
+  return t;
+}
+
 // The FP32 rates of one target block b whose rays are [r0, r1) of `rays`
 // (columns in three planes of nray), written to its cells in rates6; one
 // warp.  Phase A: per-ray parameters (ray_params_f32), one lane per ray, 32
@@ -551,37 +595,8 @@ __device__ __forceinline__ void rate_block_f32(const GridDev &g, const float4 *_
   int bix, biy, biz;
   block_cell(g, b, 0, &bix, &biy, &biz);
   for (uint64_t rc = r0; rc < r1; rc += 32) {
-    const uint64_t r = rc + lane;
-    int t = -1;
-    bool quad = false;
-    if (r < r1) {
-      const uint32_t w = __ldg(rays + r);
-      const uint32_t e = w >> 5;
-      t = (int)(w & 31u);
-      if (kServed && __ldg(pred + 6 * nray + r) != 0.f) {
-#pragma unroll
-        for (int s = 0; s < 6; s++) S.c.out[lane][s] = __ldg(pred + s * nray + r);
-      } else {
-        quad = true;
-        const int lx = bix + (t >> 4), ly = biy + ((t >> 2) & 3), lz = biz + (t & 3);
-        const float4 ep = __ldg(emit_pos + e);
-        const float4 rw = __ldg(raw + cell_index(g, lx, ly, lz));
-        const RayParams p = ray_params_f32(g, g.ix0 + lx, g.iy0 + ly, g.iz0 + lz, ep.x, ep.y, ep.z, __ldg(tau + r),
-                                           __ldg(tau + nray + r), __ldg(tau + 2 * nray + r), rw, __ldg(total + e));
-        S.c.rec[lane] = ray_rec(p, (int)e);
-#pragma unroll
-        for (int s = 0; s < 3; s++) S.c.p[lane][s] = p.P[s];
-      }
-    }
-    int nq = (int)min((uint64_t)32, r1 - rc);
-    if (kServed) {
-      const unsigned m = __ballot_sync(0xffffffffu, quad);
-      if (quad) S.q[__popc(m & ((1u << lane) - 1u))] = lane;
-      nq = __popc(m);
-    }
-    __syncwarp();
-    chunk_rates(S.c, tab, specn, kServed ? S.q : nullptr, nq, lane);
-    __syncwarp();
+    const int t = rate_chunk<kServed>(g, raw, emit_pos, specn, total, tab, bix, biy, biz, rc, r1, rays, nray, tau, S,
+                                      lane, pred);
     add_chunk_in_order(acc, lane, t, S.c.out, S.cnt, S.src);
   }
   if (own_valid) {

@@ -156,3 +156,26 @@ def test_f32_forms_and_partial_rounds(cuda_ok, edge, nsrc, depth):
     assert big[:3].any(axis=1).all()
     tau = np.log(f64.max(axis=1, keepdims=True) / np.where(big, f64, 1.0)).clip(0.0)
     assert ((np.abs(f32 - f64) / np.where(big, f64, 1.0))[big] < (2e-6 + 4 * 2.0 ** -24 * (tau + 2 * depth))[big]).all()
+
+
+@pytest.mark.parametrize("edge,nsrc", [(6, 3), (13, 40), (48, 9)])
+def test_cta_per_block_equals_warp_per_block(cuda_ok, edge, nsrc):
+    """A range of few blocks takes a CTA per block, a long one a warp per
+    block; a batch (warps) and the blocks one by one (CTAs) give the same
+    rates bit for bit."""
+    import torch
+    from argot_b200 import _lib as L, workload as W
+    from argot_b200.batch import Batch
+    wl = W.tiny(edge, nsrc, seed=edge)
+    b = Batch([wl])
+    b.configure(mode=1, parts=1)
+    b.run()
+    pb = b.problems[0]
+    g = pb.groups[0]
+    rays, tau = pb.alloc_group_buffers()
+    pb.emit(g, rays)
+    pb.march(g, rays, tau)
+    rates = torch.full((6 * pb.ncell,), float("nan"), device="cuda")
+    pb.rates(g, rays, tau, rates, L.RATE_EXACT_F32)
+    assert torch.equal(rates, b.rates[0])
+    pb.check_device_error()
