@@ -20,7 +20,7 @@
 // offset and wrap periodically, so they are translations of one path: the
 // same sequence of faces crossed and the same chords, and every cell of the
 // box is crossed by the whole sequence of one layer.  k_art_sweep forms that
-// path once per CTA (in double) and marches 256 rays along it in step; the
+// path once per CTA (in double) and marches its rays along it in step; the
 // chord length that the reference sums per cell and angle is then one number
 // per angle (the layer's thickness along the ray), so an angle's term is
 // linear in its crossings and all angles add into one accumulator per cell
@@ -63,13 +63,14 @@ struct ArtAngle {
 // Per-cell data of the march: absorption coefficients [cm^-1] and source
 // functions of the three frequencies in one 32-byte record, read with one
 // 256-bit load per step.
+// The first two frequencies' lie in pairs for the f32x2 operations.
 struct __align__(32) ArtCell {
-  float a1, a2, a3, s1, s2, s3, pad0, pad1;
+  float a1, a2, s1, s2, a3, s3, pad0, pad1;
 };
 __device__ __forceinline__ ArtCell load_cell(const ArtCell *p) {
   ArtCell c;
   asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=f"(c.a1), "=f"(c.a2), "=f"(c.a3), "=f"(c.s1), "=f"(c.s2), "=f"(c.s3), "=f"(c.pad0), "=f"(c.pad1)
+      : "=f"(c.a1), "=f"(c.a2), "=f"(c.s1), "=f"(c.s2), "=f"(c.a3), "=f"(c.s3), "=f"(c.pad0), "=f"(c.pad1)
       : "l"(p));
   return c;
 }
@@ -162,7 +163,7 @@ __global__ void __launch_bounds__(256) k_art_cells(uint64_t n, const float *__re
     const double e1 = (rec_hii_a(t) - rec_hii_b(t)) * ne * nhii * kNuLeV * kThrHI * kEVtoErg / (4.0 * kPi);
     const double e2 = (rec_heii_a(t) - rec_heii_b(t)) * ne * nheii * kNuLeV * kThrHeI * kEVtoErg / (4.0 * kPi);
     const double e3 = (rec_heiii_a(t) - rec_heiii_b(t)) * ne * nheiii * kNuLeV * kThrHeII * kEVtoErg / (4.0 * kPi);
-    const ArtCell cl{a1, a2, a3, (float)(e1 / (double)a1), (float)(e2 / (double)a2), (float)(e3 / (double)a3),
+    const ArtCell cl{a1, a2, (float)(e1 / (double)a1), (float)(e2 / (double)a2), a3, (float)(e3 / (double)a3),
                      0.f, 0.f};
     cells[c] = cl;
     if (cells_t) cells_t[transposed(c, ny, nz)] = cl;
@@ -198,9 +199,6 @@ __device__ __forceinline__ void att(float tau, float *et, float *em1) {
 // measured 8% faster than 8 (32 registers, with spills).
 #ifndef ARGOT_ART_MIN_CTAS
 #define ARGOT_ART_MIN_CTAS 6
-#endif
-#ifndef ARGOT_ART_SWEEP_CTAS
-#define ARGOT_ART_SWEEP_CTAS 5
 #endif
 // One thread per ray of angles [a0, a0 + na); acc: na planes of ncell
 // float4 (sum of I (1 - e^-tau) per frequency, chord length).  A ray that
@@ -393,42 +391,61 @@ struct ArtAxis {
   }
 };
 constexpr int kArtMaxSteps = 3072;  // steps of a path held in shared memory
-constexpr int kArtThreads = 256;
+constexpr int kArtThreads = 128, kArtCtas = 7;
 constexpr uint64_t kArtWaves = 4;
 
 // e^-tau and 1 - e^-tau from y = tau log2(e) / 2: below tau = 1, 1 - e^-tau =
 // tau e^(-tau/2) sinh(tau/2)/(tau/2) with the polynomial of the FP32 rates
 // (argot_b200/fits.py, in (2 y)^2; no cancellation, within 1.5e-7), above, the
 // difference.
-__device__ __forceinline__ void att_y(float y, float *et, float *em1) {
-  constexpr float k = 1.38629436f;  // tau = 2 ln2 y
+__device__ __forceinline__ float ex2_neg(float y) {
   float h;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(h) : "f"(-y));
-  const float v = y * y, e = h * h;
-  const float p = fmaf(v, fmaf(v, fmaf(v, k * 64.f * 3.4621803e-07f, k * 16.f * 0.000120223514f), k * 4.f * 0.0200188775f), k);
+  return h;
+}
+constexpr float kAttK = 1.38629436f;  // tau = 2 ln2 y
+constexpr float kAtt1 = kAttK * 4.f * 0.0200188775f, kAtt2 = kAttK * 16.f * 0.000120223514f,
+                kAtt3 = kAttK * 64.f * 3.4621803e-07f;
+constexpr float kAttY = 0.72134752f;  // tau = 1
+__device__ __forceinline__ void att_y(float y, float *et, float *em1) {
+  const float h = ex2_neg(y), v = y * y, e = h * h;
+  const float p = fmaf(v, fmaf(v, fmaf(v, kAtt3, kAtt2), kAtt1), kAttK);
   *et = e;
-  *em1 = y < 0.72134752f ? y * (h * p) : 1.f - e;
+  *em1 = y < kAttY ? y * (h * p) : 1.f - e;
+}
+// two at a time
+__device__ __forceinline__ void att_y2(float2 y, float2 *et, float2 *em1) {
+  const float2 h = make_float2(ex2_neg(y.x), ex2_neg(y.y)), v = __fmul2_rn(y, y), e = __fmul2_rn(h, h);
+  float2 p = __ffma2_rn(v, make_float2(kAtt3, kAtt3), make_float2(kAtt2, kAtt2));
+  p = __ffma2_rn(v, p, make_float2(kAtt1, kAtt1));
+  p = __ffma2_rn(v, p, make_float2(kAttK, kAttK));
+  const float2 lo = __fmul2_rn(y, __fmul2_rn(h, p));
+  *et = e;
+  *em1 = make_float2(y.x < kAttY ? lo.x : 1.f - e.x, y.y < kAttY ? lo.y : 1.f - e.y);
 }
 
-// What bounds the sweep at 128^3 cells / 768 directions (12.1 ms a pass; the
-// general march with its per-angle accumulators, 64 angles at a time, took
-// 33.4 ms and moved 52 GB of accumulators through DRAM): issue, 81% of the
-// cycles, then the reductions on the way to L2 (68% of that path; one per
-// crossing: 81%, 12.5 ms).  Without the copy with y fastest, the rays of the
-// faces normal to z read and reduce one line per lane: 17.0 ms.  5 CTAs per
-// SM (48 registers); 4: 12.3 ms, 6: 12.4 ms.
+// One CTA: 128 pairs of rays of one angle (blockIdx.y), marched together along
+// the angle's path.  A step's axis is the same for all rays, so a ray keeps
+// its cell index and, per side axis, the steps to its wrap.  A thread's two
+// rays start in neighbouring rows, a warp's in 32 cells of a row, a CTA's in
+// tiles of 8 rows, so that a side step finds the cells its neighbours just
+// read in L1, and the sums of a cell pass from ray to ray before they go to
+// memory.  acc[c] += (I (1 - e^-tau)) d / L per frequency, L the layer's path
+// length and d the smallest cell side (a factor of order one, so that the
+// sums keep the intensities' range).  The next step's cell is loaded before
+// this step's arithmetic.  cells_t, acc_t: the layout with y fastest for the
+// start faces normal to z, whose rays would otherwise lie a row apart (null:
+// none).
 //
-// One CTA: 256 rays of one angle (blockIdx.y), marched together along the
-// angle's path.  A step's axis is the same for all rays, so a ray keeps its
-// cell index and, per side axis, the steps to its wrap.  Rays are taken in
-// tiles of 8 rows of 32 cells of the start face, so that a side step finds
-// the cells its neighbours just read in L1.  acc[c] += (I (1 - e^-tau)) d / L
-// per frequency, L the layer's path length and d the smallest cell side (a
-// factor of order one, so that the sums keep the intensities' range).  The
-// next step's cell is loaded before this step's arithmetic.  cells_t, acc_t:
-// the layout with y fastest for the start faces normal to z, whose rays would
-// otherwise lie a row apart (null: none).
-__global__ void __launch_bounds__(kArtThreads, ARGOT_ART_SWEEP_CTAS)
+// Measured at 128^3 cells / 768 directions: 11.0 ms a pass; the general march
+// with its per-angle accumulators, 64 angles at a time, took 33.4 ms and moved
+// 52 GB of accumulators through DRAM.  On the way: one ray per thread 12.1
+// ms, one reduction per crossing 12.5 ms (the path of the reductions to L2
+// busy 81%), without the copy with y fastest 17.0 ms.  What bounds it now:
+// issue (70%), the heavy FMA pipe (55%) and the latency of the cell loads at
+// 28 warps per SM.  Launch shape: 128 threads, 7 CTAs per SM; 6: 11.1 ms, 256
+// threads x 3: 12.8 ms.
+__global__ void __launch_bounds__(kArtThreads, kArtCtas)
     k_art_sweep(ArtGeom g, const ArtAngle *__restrict__ ang, int a0, const ArtCell *__restrict__ cells,
                 float4 *__restrict__ acc, const ArtCell *__restrict__ cells_t, float4 *__restrict__ acc_t) {
   // per step: chord [cm] times log2(e) / 2, the cell index's change, 1 for a
@@ -487,76 +504,115 @@ __global__ void __launch_bounds__(kArtThreads, ARGOT_ART_SWEEP_CTAS)
                     __int_as_float(t == 1), __int_as_float(t == 2));
   }
   __syncthreads();
-  // this thread's ray: cell (ip, iq) of the start face
-  const uint32_t np = (uint32_t)nn[p], nq = (uint32_t)nn[q];
+  // this thread's rays: the cells iq of two rows of the start face, the second
+  // one's row ahead of the first's along p (row 1 of a face's odd last row: none)
+  const uint32_t np = (uint32_t)nn[p], nq = (uint32_t)nn[q], npair = (np + 1) / 2;
   const uint32_t r = blockIdx.x * kArtThreads + threadIdx.x;
-  const unsigned mask = __ballot_sync(0xffffffffu, r < np * nq);
-  if (r >= np * nq) return;
-  const uint32_t strip = r / (8u * nq), rows = min(8u, np - 8u * strip), in = r - strip * 8u * nq;
+  const unsigned mask = __ballot_sync(0xffffffffu, r < npair * nq);
+  if (r >= npair * nq) return;
+  const uint32_t strip = r / (4u * nq), rows = min(4u, npair - 4u * strip), in = r - strip * 4u * nq;
   const uint32_t chunk = in / (32u * rows), cols = min(32u, nq - 32u * chunk), at = in - chunk * 32u * rows;
-  const uint32_t ip = 8u * strip + at / cols, iq = 32u * chunk + at % cols;
-  uint32_t pos = (uint32_t)(ip * st[p] + iq * st[q] + (o[ax] > 0.0 ? 0 : (nn[ax] - 1) * st[ax]));
-  int wp = o[p] > 0.0 ? (int)(np - ip) : (int)ip + 1, wq = o[q] > 0.0 ? (int)(nq - iq) : (int)iq + 1;
+  const uint32_t ip = 2u * (4u * strip + at / cols), iq = 32u * chunk + at % cols;
+  const bool two = ip + 1 < np, swap = two && o[p] < 0.0;
+  uint32_t pos[2];
+  int wp[2], wq = o[q] > 0.0 ? (int)(nq - iq) : (int)iq + 1;
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    const uint32_t i = ip + (uint32_t)(two && (j == 1) != swap);
+    pos[j] = (uint32_t)(i * st[p] + iq * st[q] + (o[ax] > 0.0 ? 0 : (nn[ax] - 1) * st[ax]));
+    wp[j] = o[p] > 0.0 ? (int)(np - i) : (int)i + 1;
+  }
   const float il = (float)(fmin(dd[0], fmin(dd[1], dd[2])) / B.T);  // d / L
-  // the lane whose ray runs one cell ahead along q, the same row's next cell in
+  // the lane whose rays run one cell ahead along q, the same row's next cell in
   // that direction (periodically: the rays keep their distance), and whether
   // there is a lane one cell behind
   const int lane = threadIdx.x & 31, dir = o[q] > 0.0 ? 1 : -1;
-  const bool next_in_row = at % cols + 1 < cols, prev_in_row = at % cols > 0;
-  const bool has_ahead = dir > 0 ? next_in_row && lane < 31 && (mask >> (lane + 1) & 1u) : prev_in_row && lane > 0;
-  const bool has_behind = dir > 0 ? prev_in_row && lane > 0 : next_in_row && lane < 31 && (mask >> (lane + 1) & 1u);
+  const bool next_in_row = at % cols + 1 < cols && lane < 31 && (mask >> (lane + 1) & 1u);
+  const bool prev_in_row = at % cols > 0 && lane > 0;
+  const bool has_ahead = dir > 0 ? next_in_row : prev_in_row, has_behind = dir > 0 ? prev_in_row : next_in_row;
   const int ahead = has_ahead ? lane + dir : lane;
-  float m1 = 0.f, m2 = 0.f, m3 = 0.f;  // sums of the current cell not yet added to acc
-  float i1 = 0.f, i2 = 0.f, i3 = 0.f;  // intensities
-  ArtCell cl = load_cell(cells + pos);
+  // sums of the current cells not yet added to acc and intensities, of the
+  // first two frequencies and of the third
+  float2 m12[2] = {}, i12[2] = {};
+  float m3[2] = {}, i3[2] = {};
+  ArtCell cl[2] = {load_cell(cells + pos[0]), load_cell(cells + pos[1])};
+  auto flush = [&](int j) {
+    atomicAdd(acc + pos[j], make_float4(m12[j].x * il, m12[j].y * il, m3[j] * il, 0.f));
+  };
 #pragma unroll 2
   for (int k = 0; k < nstep; k++) {
     const float4 step = s_path[k];
-    const bool along_q = __any_sync(mask, __float_as_int(step.w));  // (uniform, known to the compiler as such)
-    uint32_t nxt = pos + __float_as_uint(step.y);
-    bool wrapped = false;
-    wp -= __float_as_int(step.z);
-    wq -= __float_as_int(step.w);
-    if (wp == 0 || wq == 0) {
-      wrapped = true;
-      if (wp == 0) {
-        nxt -= np * dp;
-        wp = (int)np;
-      } else {
-        nxt -= nq * dq;
+    // (uniform, known to the compiler as such)
+    const bool along_p = __any_sync(mask, __float_as_int(step.z)), along_q = __any_sync(mask, __float_as_int(step.w));
+    uint32_t nxt[2];
+    bool wrapped[2] = {false, false};
+#pragma unroll
+    for (int j = 0; j < 2; j++) nxt[j] = pos[j] + __float_as_uint(step.y);
+    if (along_p) {
+#pragma unroll
+      for (int j = 0; j < 2; j++)
+        if (--wp[j] == 0) {
+          nxt[j] -= np * dp;
+          wp[j] = (int)np;
+          wrapped[j] = true;
+        }
+    } else if (along_q) {
+      if (--wq == 0) {
+        nxt[0] -= nq * dq;
+        nxt[1] -= nq * dq;
         wq = (int)nq;
+        wrapped[0] = wrapped[1] = true;
       }
     }
-    // (past the last step the ray has left through the far face)
-    const ArtCell cn = load_cell(cells + (k + 1 < nstep ? nxt : pos));
+    // (past the last step the rays have left through the far face)
+    const bool more = k + 1 < nstep;
+    const ArtCell cn[2] = {load_cell(cells + (more ? nxt[0] : pos[0])), load_cell(cells + (more ? nxt[1] : pos[1]))};
     const float c = step.x;
     if (c > 0.f) {
-      float et, em;
-      att_y(cl.a1 * c, &et, &em);
-      m1 = fmaf(i1, em, m1);
-      i1 = fmaf(i1, et, cl.s1 * em);
-      att_y(cl.a2 * c, &et, &em);
-      m2 = fmaf(i2, em, m2);
-      i2 = fmaf(i2, et, cl.s2 * em);
-      att_y(cl.a3 * c, &et, &em);
-      m3 = fmaf(i3, em, m3);
-      i3 = fmaf(i3, et, cl.s3 * em);
+#pragma unroll
+      for (int j = 0; j < 2; j++) {
+        float2 et2, em2;
+        att_y2(__fmul2_rn(make_float2(cl[j].a1, cl[j].a2), make_float2(c, c)), &et2, &em2);
+        m12[j] = __ffma2_rn(i12[j], em2, m12[j]);
+        i12[j] = __ffma2_rn(i12[j], et2, __fmul2_rn(make_float2(cl[j].s1, cl[j].s2), em2));
+        float et, em;
+        att_y(cl[j].a3 * c, &et, &em);
+        m3[j] = fmaf(i3[j], em, m3[j]);
+        i3[j] = fmaf(i3[j], et, cl[j].s3 * em);
+      }
     }
-    // leaving along q, the ray enters the cell of the lane ahead, whose sums
-    // it takes over; else, and where no lane follows, the sums go to memory
+    // The rays enter new cells.  Along q the lane ahead was there, along p the
+    // thread's second ray: its sums are taken over.  Sums that no ray takes
+    // over go to memory.
     if (along_q) {
-      if (!has_behind) atomicAdd(acc + pos, make_float4(m1 * il, m2 * il, m3 * il, 0.f));
-      m1 = __shfl_sync(mask, m1, ahead);
-      m2 = __shfl_sync(mask, m2, ahead);
-      m3 = __shfl_sync(mask, m3, ahead);
-      if (!has_ahead) m1 = m2 = m3 = 0.f;
+      if (!has_behind) {
+        flush(0);
+        if (two) flush(1);
+      }
+#pragma unroll
+      for (int j = 0; j < 2; j++) {
+        const float a = __shfl_sync(mask, m12[j].x, ahead), b = __shfl_sync(mask, m12[j].y, ahead),
+                    d = __shfl_sync(mask, m3[j], ahead);
+        m12[j] = has_ahead ? make_float2(a, b) : make_float2(0.f, 0.f);
+        m3[j] = has_ahead ? d : 0.f;
+      }
     } else {
-      atomicAdd(acc + pos, make_float4(m1 * il, m2 * il, m3 * il, 0.f));
-      m1 = m2 = m3 = 0.f;
+      flush(0);
+      if (!along_p && two) flush(1);
+      m12[0] = along_p && two ? m12[1] : make_float2(0.f, 0.f);
+      m3[0] = along_p && two ? m3[1] : 0.f;
+      m12[1] = make_float2(0.f, 0.f);
+      m3[1] = 0.f;
     }
-    if (wrapped) i1 = i2 = i3 = 0.f;
-    pos = nxt;
-    cl = cn;
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      if (wrapped[j]) {
+        i12[j] = make_float2(0.f, 0.f);
+        i3[j] = 0.f;
+      }
+      pos[j] = nxt[j];
+      cl[j] = cn[j];
+    }
   }
 }
 
@@ -867,8 +923,10 @@ int art_run(const argot_b200_art *a, const ArtGeom &g, double denstonh, double u
   // groups of angles per launch: enough CTAs for kArtWaves fills of the GPU
   // and at least 128 angles; between groups the sums (of about 2 terms per
   // angle) go into compensated totals
-  const uint32_t tiles = (face_max + kArtThreads - 1) / kArtThreads;
-  const int group = (int)std::max<uint64_t>(128, (kArtWaves * 148 * ARGOT_ART_SWEEP_CTAS + tiles - 1) / tiles);
+  const uint64_t pairs = std::max<uint64_t>((uint64_t)((g.nx + 1) / 2) * std::max(g.ny, g.nz),
+                                            (uint64_t)((g.ny + 1) / 2) * g.nz);
+  const uint32_t tiles = (uint32_t)((pairs + kArtThreads - 1) / kArtThreads);
+  const int group = (int)std::max<uint64_t>(128, (kArtWaves * 148 * kArtCtas + tiles - 1) / tiles);
   int in_group = 0;
   for (int i = 0, left = nswept; left > 0; i = run_end(i)) {
     if (steps(i) == 0) continue;

@@ -140,27 +140,28 @@ __global__ void __launch_bounds__(256) k_walk(GridDev g, const DevNode *__restri
 // Which blocks run at the same time decides where the gathers hit: warps
 // work through their emitters in the same depth-first order, so blocks that
 // lie together walk the same cells.  Blocks are therefore taken in tiles
-// (block_of_item): the 32 warps of a CTA hold 2 x 4 x 4 blocks (4 x 16 x 16
+// (block_of_item): two CTAs of 16 warps hold 2 x 4 x 4 blocks (4 x 16 x 16
 // cells), consecutive CTAs 8 x 8 x 8 blocks, instead of a row of blocks along
 // z.  ncu, 224^3 cells / 32 sources: L1 sector hits 37% -> 56%, L2 63% -> 89%,
 // DRAM no longer read 64 GB per launch, 82.9 -> 72.5 ms; 256^3 / 1024
-// clustered sources: 0.697 s -> 0.610 s (CTAs of 8 warps in tiles 0.664 s, of
-// 16 warps 0.629 s).  What bounds it now: the L1 data pipe (77% of its peak,
+// clustered sources: 0.697 s -> 0.610 s with CTAs of 32 warps, 0.629 s with 16,
+// 0.664 s with 8; but the step that runs it beside the rates takes 0.990,
+// 0.975 and 0.983 s, so 16.  What bounds it now: the L1 data pipe (77% of its peak,
 // one line per cycle for each quarter warp of a 16-byte gather), the ALU
 // (68%) and issue (71%) together.
-// Launch shape: 64 warps per SM (32 registers) in CTAs of 32 warps.  A range
+// Launch shape: 64 warps per SM (32 registers) in CTAs of 16 warps.  A range
 // of few blocks is cut finer: each block's chunks of 32 rays into segments,
 // one warp each, until there are kMarchItems items per warp slot (32^3 cells
 // / 8 sources: 78 -> 41 us, 64^3 / 16: 0.49 -> 0.45 ms; more items per slot
-// on larger meshes: no change), in CTAs of 8 warps where 32 would leave SMs
-// empty.  What lives across a ray's walk is kept out of
+// on larger meshes: no change), in CTAs of 8 warps where those would leave
+// warp slots empty.  What lives across a ray's walk is kept out of
 // registers: the Kahan columns in per-thread shared-memory slots, the
 // block's state (item, ray count, packed coordinates, first ray; the same
 // for the warp's lanes) in per-warp shared memory, read back after each ray.
 // kInside: every emitter lies inside the box (the host checks the emitters'
 // bounding box), so rays start at their emitter and the launch contains no
 // call.
-constexpr int kMarchWide = 1024, kMarchNarrow = 256;
+constexpr int kMarchWide = 512, kMarchNarrow = 256;
 constexpr uint64_t kMarchItems = 2;
 
 // One level of a tiled enumeration of nx * ny * nz blocks (tiles of tx * ty *
