@@ -454,8 +454,7 @@ int argot_b200_dev_tree_upload(const argot_b200_tree *t, argot_b200_dev_tree **o
     for (int k = 0; k < kNu; k++) s += spec[e * kNu + k];
     total[e] = s;
     const double inv = s > 0.0 ? 1.0 / s : 0.0;
-    // bin-pair order of the packed rate loop: position 2 p + h holds bin
-    // (p % 8) + 16 (p / 8) + 8 h (spec_lane_index)
+    // in the lane order of the FP32 rate loop (spec_lane_index)
     for (int k = 0; k < kNu; k++) specn[e * kNu + spec_lane_index(k)] = (float)(spec[e * kNu + k] * inv);
   }
   cudaError_t err = cudaSuccess;

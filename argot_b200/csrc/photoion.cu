@@ -124,9 +124,8 @@ __global__ void __launch_bounds__(32 * kF32Warps, ARGOT_RATE_MIN_CTAS)
 // them in order, two of the six rates each (the same sums, bit for bit).
 // Measured against one warp per block: 32^3 cells / 8 sources (1024 blocks of
 // 200 rays) 110 -> 88 us, 48^3 / 64 (3456 blocks of 1460) 1.54 -> 1.32 ms;
-// 64^3 / 16 (8192 of
-// 420) 0.94 against 0.82 ms, the warps' waits outweighing the better split:
-// hence the line at two blocks per warp slot.
+// 64^3 / 16 (8192 of 420) 0.94 against 0.82 ms, the warps' waits outweighing
+// the better split: hence the line at two blocks per warp slot.
 struct CellSumPair {
   float (*a)[32];
   int lane, q0;

@@ -24,7 +24,7 @@
 //     centre are the host's flat sums over the sources in input order (the
 //     centre weighted by the first bin).
 //  6. The emitter table (nodes, then sources in input order): positions,
-//     FP64 spectra, totals and the normalised FP32 spectra in bin-pair
+//     FP64 spectra, totals and the normalised FP32 spectra in lane
 //     order, and the emitters' bounding box.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
@@ -221,7 +221,7 @@ __global__ void k_root_sums(int n, const float *__restrict__ pos, const double *
 }
 
 // The emitter table: emitter e < nn is node e, else source e - nn (input
-// order).  total = sum of the bins in order; specn in bin-pair order.
+// order).  total = sum of the bins in order; specn in lane order.
 __global__ void k_emitters(int nn, int n, const DevNode *__restrict__ nodes, const float *__restrict__ pos,
                            const double *__restrict__ spec, float4 *__restrict__ epos,
                            double *__restrict__ espec, float *__restrict__ especn, double *__restrict__ etot) {

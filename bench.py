@@ -892,9 +892,13 @@ def run_art(args):
     total = allsum(ws, float(steps_per_pass) * args.steps, dev)
     hbm, _, peak_kind = measured_peaks()
     # algorithmic bytes of one pass: per step two float4 of cell data read
-    # and one float4 reduction; per cell and direction one float4 folded;
-    # per cell 8 planes in, 6 planes of totals and 6 rate planes
-    alg = 48.0 * steps_per_pass + 16.0 * n * art.nang + 4.0 * n * (8 + 6 + 12)
+    # and one float4 reduction (from and to L2); per cell 8 planes in, 6
+    # planes of totals and 6 rate planes
+    alg = 48.0 * steps_per_pass + 4.0 * n * (8 + 6 + 12)
+    # launches: cells, the sweeps of the directions in groups with a gather
+    # between two, the closing kernel (csrc/art.cu art_run)
+    tiles = -(-((wl.edge + 1) // 2 * wl.edge) // 128)
+    groups = -(-art.nang // max(128, -(-4 * 148 * 7 // tiles)))
     achieved = alg / (t / args.steps) / 1e9
     # e2e: the 8 planes from pinned host memory, the pass, the rates back
     pin_f = torch.from_numpy(planes).pin_memory()
@@ -920,16 +924,16 @@ def run_art(args):
         "data": "synthetic (seeded lognormal mesh, ionisation around clustered sources)",
         "config": {"workload": f"art on {wl.name}", "mesh": f"{wl.edge}^3", "directions": art.nang,
                    "angles_per_pass": apass, "steps_per_pass": steps_per_pass,
-                   "l2": "cell data 1 GB at 256^3, 67 MB at 128^3; accumulators larger than L2; no flush",
+                   "l2": "cell data 1 GB at 256^3, 134 MB at 128^3 (both layouts); no flush",
                    "parallelism": f"{ws} independent meshes (one per GPU)"},
-        "roofline": {"kernel": "k_art_cells + k_art_trace + k_art_fold (one pass)", "bound": "hbm",
+        "roofline": {"kernel": "k_art_cells + k_art_sweep + k_art_gather + k_art_close (one pass)", "bound": "hbm",
                      "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                      "peak_kind": f"{peak_kind} hbm_gbs", "traffic": None,
-                     "bytes_model": "48 B per ray-cell step + 16 B per cell and direction + 104 B per cell"},
+                     "bytes_model": "48 B per ray-cell step (served by L1 and L2) + 104 B per cell"},
         "e2e": {"value": float(steps_per_pass) / te, "unit": UNIT, "h2d_bytes_per_step": int(planes.nbytes),
                 "d2h_bytes_per_step": int(6 * n * 4), "s_per_step": te},
         "clocks": clk,
-        "gpu_launches": (2 + 2 * ((art.nang + apass - 1) // apass)) * args.steps,
+        "gpu_launches": (2 + 2 * groups - 1) * args.steps,
     }
     if rank == 0 and ws == 1 and not args.no_cpu_baseline:
         try:
