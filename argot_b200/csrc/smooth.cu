@@ -10,6 +10,8 @@
 // double, stored as float.  At the mesh faces: a copy of the nearest cell
 // (the reference's default build, `isolated = yes`, with no neighbour rank)
 // or the periodic image.  Bit-identical to the reference.
+#include <algorithm>
+
 #include "march.cuh"
 
 namespace argot {
@@ -124,16 +126,75 @@ __global__ void __launch_bounds__(kSmoothThreads, 4)
   }
 }
 
+// The same with one thread per cell and no sharing between cells: 27 loads
+// per cell and plane, but no lane without a cell on a thin mesh.
+template <bool kIsolated>
+__global__ void __launch_bounds__(256)
+    k_smooth_flat(int nx, int ny, int nz, const float *__restrict__ in, float *__restrict__ out, int nplanes) {
+  const uint64_t ncell = (uint64_t)nx * ny * nz;
+  const double kNormal = 1.0 / (30.0 + 26.0);
+  for (uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < ncell;
+       c += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t row = (uint32_t)c / (uint32_t)nz, ix = row / (uint32_t)ny;
+    const int at[3] = {(int)ix, (int)(row - ix * (uint32_t)ny), (int)((uint32_t)c - row * (uint32_t)nz)};
+    uint32_t jx[3], jy[3], jz[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      jx[a] = (uint32_t)face_index<kIsolated>(at[0] + a - 1, nx);
+      jy[a] = (uint32_t)face_index<kIsolated>(at[1] + a - 1, ny);
+      jz[a] = (uint32_t)face_index<kIsolated>(at[2] + a - 1, nz);
+    }
+    uint32_t off[27];
+#pragma unroll
+    for (int k = 0; k < 27; k++)
+      off[k] = (jx[k / 9] * (uint32_t)ny + jy[k / 3 % 3]) * (uint32_t)nz + jz[k % 3];
+#pragma unroll 1
+    for (int s = 0; s < nplanes; s++) {
+      const float *__restrict__ f = in + s * ncell;
+      float acc = __ldg(f + off[0]);
+#pragma unroll
+      for (int k = 1; k < 13; k++) acc = __fadd_rn(acc, __ldg(f + off[k]));
+      double d = __dadd_rn((double)acc, __dmul_rn(30.0, (double)__ldg(f + off[13])));
+#pragma unroll
+      for (int k = 14; k < 27; k++) d = __dadd_rn(d, (double)__ldg(f + off[k]));
+      out[s * ncell + c] = __double2float_rn(__dmul_rn(kNormal, d));
+    }
+  }
+}
+
+// Which kernel a mesh takes.  k_smooth's time goes with the slots it fills,
+// lanes with or without a cell: fills of the GPU (kSmoothWarps warps per SM)
+// times the planes a warp steps through, two of them read ahead, times 64
+// cells per warp.  On a thin mesh (few cells along z or y, one plane along
+// x) most slots hold no cell.  The line lies at kSlotsPerCell slots per cell
+// (measured over 290 meshes: 512 x 512 x 4 195 us in runs against 58 us flat,
+// 256 x 256 x 14 53 and 50, 256 x 256 x 16 53 and 54, 256 x 256 x 33 123 and 134);
+// up to kFewSteps plane steps in all, both take about 10 us.
+constexpr uint64_t kSmoothWarps = 16, kFewSteps = 16;
+constexpr double kSlotsPerCell = 2.9;
+
 // Smooths nplanes planes of ncell floats (in -> out).
 int launch_smooth_planes(int nx, int ny, int nz, const float *in, float *out, int nplanes, int isolated,
                          cudaStream_t st) {
   const uint64_t ncell = (uint64_t)nx * ny * nz;
   if (!ncell || nplanes <= 0) return 0;
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // shorter segments where the mesh would leave the GPU's warps idle
-  const uint64_t columns = (uint64_t)((ny + 1) / 2) * ((nz + 31) / 32);
+  const uint64_t columns = (uint64_t)((ny + 1) / 2) * ((nz + 31) / 32), slots = kSmoothWarps * sms;
   int run = kRun;
-  while (run > 3 && columns * ((nx + run - 1) / run) * (uint64_t)nplanes < 148 * 16) run /= 2;
+  while (run > 3 && columns * ((nx + run - 1) / run) * (uint64_t)nplanes < slots) run /= 2;
   const uint64_t warps = columns * ((nx + run - 1) / run);
+  const uint64_t steps = (warps * nplanes + slots - 1) / slots * (std::min(run, nx) + 2);
+  if (steps > kFewSteps && (double)(steps * slots * 64) > kSlotsPerCell * (double)ncell * nplanes) {
+    const unsigned blocks = (unsigned)std::min<uint64_t>((ncell + 255) / 256, (uint64_t)sms * 8);
+    if (isolated)
+      k_smooth_flat<true><<<blocks, 256, 0, st>>>(nx, ny, nz, in, out, nplanes);
+    else
+      k_smooth_flat<false><<<blocks, 256, 0, st>>>(nx, ny, nz, in, out, nplanes);
+    ARGOT_CUDA_TRY(cudaGetLastError());
+    return 0;
+  }
   const dim3 grid((unsigned)((warps + kSmoothThreads / 32 - 1) / (kSmoothThreads / 32)), (unsigned)nplanes);
   if (isolated)
     k_smooth<true><<<grid, kSmoothThreads, 0, st>>>(nx, ny, nz, run, in, out);

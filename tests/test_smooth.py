@@ -152,16 +152,9 @@ def test_dropin_smooth_photoion_rate(cuda_ok, edge, isolated):
         lib.argot_b200_set_dropin_smooth_faces(1)
 
 
-@pytest.mark.gpu
-@pytest.mark.parametrize("isolated", [True, False])
-@pytest.mark.parametrize("n", [(1, 1, 1), (2, 3, 33), (7, 1, 64), (25, 6, 31), (49, 4, 97), (30, 5, 32), (3, 2, 1)])
-def test_device_smoothing_ragged(cuda_ok, n, isolated):
-    """Meshes whose axes are no multiple of the kernel's rows, segments and
-    32 cells along z, with zeros, subnormals and infinities among the rates:
-    the same bits as the restatement."""
-    import torch
-    from argot_b200 import _lib as L
-    import ctypes as C
+def _ragged_planes(n, isolated):
+    """Six planes with zeros, subnormals and an infinity, and their smoothing
+    in the reference's order of sums."""
     rng = np.random.default_rng(sum(n))
     x = (10.0 ** rng.normal(-12, 3, (6,) + n)).astype(np.float32)
     x[0, rng.random(n) < 0.2] = 0.0
@@ -179,9 +172,69 @@ def test_device_smoothing_ragged(cuda_ok, n, isolated):
         for t in terms[14:]:
             d = d + t.astype(np.float64)
         want[s] = (SM.NORMAL * d).astype(np.float32)
+    return x, want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("isolated", [True, False])
+@pytest.mark.parametrize("n", [(1, 1, 1), (2, 3, 33), (7, 1, 64), (25, 6, 31), (49, 4, 97), (30, 5, 32), (3, 2, 1)])
+def test_device_smoothing_ragged(cuda_ok, n, isolated):
+    """Meshes whose axes are no multiple of the kernel's rows, segments and
+    32 cells along z, with zeros, subnormals and infinities among the rates:
+    the same bits as the restatement."""
+    import torch
+    from argot_b200 import _lib as L
+    import ctypes as C
+    x, want = _ragged_planes(n, isolated)
     g = L.Grid(*n, 0, 0, 0, 0.0, 0.0, 0.0, *map(float, n), 0.0, 0.0, 0.0, 1.0, 1.0, 1.0, 1.0, 1.0)
     xin = torch.from_numpy(x.ravel().copy()).cuda()
     out = torch.full_like(xin, -1.0)
     L.check(L.load().argot_b200_smooth_rates(C.byref(g), xin.data_ptr(), out.data_ptr(), int(isolated),
                                              torch.cuda.current_stream().cuda_stream), "smooth_rates")
     assert np.array_equal(out.cpu().numpy().reshape(want.shape), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("isolated", [True, False])
+@pytest.mark.parametrize("n", [(20000, 1, 1), (1, 9000, 3), (700, 3, 5), (150, 150, 4), (1, 300, 300), (2, 300, 300),
+                               (96, 96, 15), (96, 96, 17)])
+def test_device_smoothing_thin(cuda_ok, n, isolated):
+    """Meshes on both sides of the line between the two kernels: the same
+    bits as the restatement."""
+    import torch
+    from argot_b200 import _lib as L
+    import ctypes as C
+    x, want = _ragged_planes(n, isolated)
+    g = L.Grid(*n, 0, 0, 0, 0.0, 0.0, 0.0, *map(float, n), 0.0, 0.0, 0.0, 1.0, 1.0, 1.0, 1.0, 1.0)
+    xin = torch.from_numpy(x.ravel().copy()).cuda()
+    out = torch.full_like(xin, -1.0)
+    L.check(L.load().argot_b200_smooth_rates(C.byref(g), xin.data_ptr(), out.data_ptr(), int(isolated),
+                                             torch.cuda.current_stream().cuda_stream), "smooth_rates")
+    assert np.array_equal(out.cpu().numpy().reshape(want.shape), want)
+
+
+@pytest.mark.gpu
+def test_thin_mesh_costs_its_cells(cuda_ok):
+    """A mesh of four cells along z takes no longer than one of four times as
+    many cells with full rows (measured 58 us and 142 us)."""
+    import torch
+    from argot_b200 import _lib as L
+    import ctypes as C
+    lib, st = L.load(), torch.cuda.current_stream().cuda_stream
+
+    def run(n):
+        g = L.Grid(*n, 0, 0, 0, 0.0, 0.0, 0.0, *map(float, n), 0.0, 0.0, 0.0, 1.0, 1.0, 1.0, 1.0, 1.0)
+        x = torch.rand(6 * n[0] * n[1] * n[2], device="cuda")
+        out = torch.empty_like(x)
+        times = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(5):
+                L.check(lib.argot_b200_smooth_rates(C.byref(g), x.data_ptr(), out.data_ptr(), 1, st), "smooth_rates")
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    assert run((512, 512, 4)) < run((256, 256, 64))
