@@ -142,6 +142,41 @@ __device__ __forceinline__ void rate_bins_f64(const RayCols &c, const double *__
   }
 }
 
+// The same over all bins and species with the reference's operations in its
+// order, for rays whose columns or rates are not finite (a source at the
+// target's centre, an infinite or undefined field): which of the rates are
+// then infinite and which undefined depends on every operation.
+static __device__ __noinline__ void rate_bins_f64_in_order(const RayCols &c, const double *__restrict__ spec,
+                                                           double out[6]) {
+  const double thr[3] = {kThrHI, kThrHeI, kThrHeII};
+  double G[3] = {0.0, 0.0, 0.0}, H[3] = {0.0, 0.0, 0.0};
+#pragma unroll 1
+  for (int k = 0; k < kNu; k++) {
+    double cs[3], d[3];
+#pragma unroll
+    for (int s = 0; s < 3; s++) {
+      cs[s] = c_tab64.cs[k][s];
+      d[s] = __dmul_rn(c.dN[s], cs[s]);
+    }
+    const double tau = __dadd_rn(__dadd_rn(__dmul_rn(c.N[0], cs[0]), __dmul_rn(c.N[1], cs[1])),
+                                 __dmul_rn(c.N[2], cs[2]));
+    const double dtot = __dadd_rn(d[0], __dadd_rn(d[1], d[2]));
+    const double pabs = __dmul_rn(__dmul_rn(__ldg(spec + k), exp(-tau)), __dsub_rn(1.0, exp(-dtot)));
+    const double den = __dadd_rn(dtot, kTiny), v = (double)c_tab.nu_f[k];
+#pragma unroll
+    for (int s = 0; s < 3; s++) {
+      const double w = __dmul_rn(__ddiv_rn(d[s], den), pabs);
+      G[s] = __dadd_rn(G[s], __dmul_rn(w, c.rN[s]));
+      if (v > thr[s]) H[s] = __dadd_rn(H[s], __dmul_rn(__dmul_rn(w, __dsub_rn(v, thr[s])), c.rN[s]));
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < 3; s++) {
+    out[s] = G[s];
+    out[3 + s] = __dmul_rn(H[s], kHNuL);
+  }
+}
+
 // The rates of a ray: out[0..2] Gamma, out[3..5] Heat.  75^3 cells, 24 sources
 // (the step with the reference-order march): 27.5 ms with three divisions a bin,
 // 17.1 ms now; bound by the FP64 operations of the two exponentials.
@@ -151,12 +186,15 @@ static __device__ __noinline__ void rate_bins_f64(const RayCols &c, const double
   rate_bins_f64<1>(c, spec, 0, k1, G, H);
   rate_bins_f64<2>(c, spec, k1, k2, G, H);
   rate_bins_f64<3>(c, spec, k2, kNu, G, H);
+  double all = 0.0;
 #pragma unroll
   for (int s = 0; s < 3; s++) {
     const double f = c.dN[s] * c.rN[s];
     out[s] = f * G[s];
     out[3 + s] = f * H[s] * kHNuL;
+    all += ((c.N[s] + c.dN[s]) + c.rN[s]) + (out[s] + out[3 + s]);
   }
+  if (!isfinite(all)) rate_bins_f64_in_order(c, spec, out);
 }
 
 __device__ __forceinline__ float ex2_approx(float x) {

@@ -179,3 +179,35 @@ def test_cta_per_block_equals_warp_per_block(cuda_ok, edge, nsrc):
     pb.rates(g, rays, tau, rates, L.RATE_EXACT_F32)
     assert torch.equal(rates, b.rates[0])
     pb.check_device_error()
+
+
+@pytest.mark.parametrize("what", ["centre", "inf", "nan", "zeros"])
+def test_exact_f64_odd_fields(cuda_ok, oracle, what):
+    """A source at a cell's centre, an infinite or undefined field, cells
+    without a species: the rates that the reference's operations leave
+    infinite or undefined are so here too, the others agree."""
+    from argot_b200 import workload as W
+    from argot_b200 import _lib as L
+    from gpu_util import run_problem, ray_segments
+    from oracle.oracle import unit_box_grid
+    wl = W.plain(8, 3, seed=2)
+    if what == "centre":
+        wl.src_pos[0] = (3.5 / 8, 4.5 / 8, 2.5 / 8)
+    elif what == "inf":
+        wl.dens[37] = np.inf
+    elif what == "nan":
+        wl.fHeI[101] = np.nan
+    else:
+        wl.dens[::3] = 0.0
+        wl.fHI[::5] = 0.0
+        wl.fHeII[1::2] = 0.0
+    pb, emit, tgt, tau, rates = run_problem(wl, L.PRECISION_REFERENCE, L.RATE_EXACT_F64)
+    segs = ray_segments(pb, emit, tgt)
+    with np.errstate(all="ignore"):
+        want = oracle.photoion_f64ref(unit_box_grid(8, wl.lunit, wl.denstonh), wl.fields(), tau, tgt, segs[:, :3],
+                                      _ref_spectra(pb, emit))
+    assert np.array_equal(np.isnan(rates), np.isnan(want))
+    assert np.array_equal(np.isinf(rates), np.isinf(want))
+    ok = np.isfinite(want)
+    assert ok.all() == (what == "zeros")
+    assert (np.abs(rates[ok] - want[ok]) <= F64_RTOL * np.abs(want[ok])).all()
