@@ -274,10 +274,10 @@ __device__ __forceinline__ RayParams ray_params_f32(const GridDev &g, int gix, i
 // Stage 0 ends below the HeII threshold (bin 102), so it has no HeII terms;
 // they would add exact zeros.
 //
-// What bounds it: the heavy FMA pipe.  A ray takes 62 to 66 packed
-// operations at 2.1 cycles (f32x2 operations issue on that pipe only) and
-// about a dozen scalar ones, 150 cycles of the 205 it takes per SM
-// sub-partition.  Before, four 8-lane groups per warp integrated two rays
+// What bounds it: the heavy FMA pipe.  A ray takes 62 and 64 packed
+// operations in the two thin forms, 69 in form 2 and 70 to 72 beyond, at 2.1 cycles
+// (f32x2 operations issue on that pipe only) and about a dozen scalar ones:
+// about 150 cycles of the 205 it takes per SM sub-partition, counted from the code.  Before, four 8-lane groups per warp integrated two rays
 // each and read every bin pair's 48-byte table entry from shared memory and
 // its spectrum from global memory: 145 instructions and 41 L1 data-pipe
 // cycles per ray (63% of that pipe, of which the march beside it needs 77%)
@@ -329,10 +329,17 @@ __device__ __forceinline__ float2 sinhc_half2(float2 dl) {
 // How the stages of a ray with cell columns D form the factor: 0 thin, 1
 // the degree-3 polynomial, 2 the SFU form for the bins at or above kPhiXMax
 // and the polynomial for the others.  Stage m's x is at most sum_s D_s max
-// sigma_s over its bins and those above (smax).  Four forms of the whole ray
-// are compiled, the cheapest that holds is taken: its stages' forms are
-// 0: 1 0 0 0, 1: 1 1 0 0, 2: 2 1 1 1, 3: 2 2 2 2.  The choice depends on the
-// ray alone, and a ray has the warp to itself, so the branch is uniform.
+// sigma_s over its bins and those above (smax), so it falls from stage to
+// stage.  Four forms of the whole ray are compiled, the cheapest that holds
+// is taken: its stages' forms are 0: 1 0 0 0, 1: 1 1 0 0, 2: 2 1 1 1 and, from 3
+// on, 2 2 2 2 where stage 2 takes the SFU form from 4 on and stage 3 with 5
+// only (a branch in the loop; each of the three compiled by itself cost the
+// other forms 2%).  The choice depends on the ray alone, and a ray has the
+// warp to itself, so the branches are uniform.
+// Measured at 64^3 cells / 16 sources, cells of optical depth 0.5, 2, 7, 20
+// and 1000 at the HI edge: 779, 875, 1040, 1041 and 1279 us; with all stages in
+// the SFU form once stage 1 needs it 775, 879, 1259, 1258 and 1262 us, with the
+// table in shared memory and eight lanes per ray 856, 922, 1021, 1085, 1368 us.
 __device__ __forceinline__ int ray_form(float D0, float D1, float D2) {
   int f[kStages];
 #pragma unroll
@@ -340,9 +347,8 @@ __device__ __forceinline__ int ray_form(float D0, float D1, float D2) {
     const float x = fmaf(D0, c_tab.smax[0][m], fmaf(D1, c_tab.smax[1][m], D2 * c_tab.smax[2][m]));
     f[m] = x >= kPhiXMax ? 2 : x < kPhiXThin ? 0 : 1;
   }
-  if (max(f[1], max(f[2], f[3])) == 2) return 3;
-  if (f[0] == 2 || f[2] || f[3]) return 2;
-  return f[1];
+  if (f[1] == 2) return f[3] == 2 ? 5 : f[2] == 2 ? 4 : 3;
+  return f[0] == 2 || f[2] || f[3] ? 2 : f[1];
 }
 
 // A ray as the loop reads it: n = the negated mid-cell columns
@@ -368,11 +374,11 @@ __device__ __forceinline__ RayRec ray_rec(const RayParams &p, int e) {
 
 // Stage m of one ray: the lane's two bins.  kNS: species with non-zero cross
 // sections; kForm as in ray_form.  ntm = -(tau + x / 2) log2(e), w = s 2^ntm
-// sinh(x/2)/(x/2) or, with kForm 2 and x >= kPhiXMax, s 2^(ntm + dl/2)
+// sinh(x/2)/(x/2) or, with kForm 2, sfu and x >= kPhiXMax, s 2^(ntm + dl/2)
 // (1 - 2^-dl) / x.
 template <int m, int kNS, int kForm>
 __device__ __forceinline__ void rate_stage(const RateLane &t, float2 s, const float2 (&n)[3], const float2 (&d)[3],
-                                           float2 (&acc)[6]) {
+                                           float2 (&acc)[6], bool sfu = true) {
   float2 ntm = __fmul2_rn(n[kNS - 1], t.l2e[m][kNS - 1]);
   float2 dl = __fmul2_rn(d[kNS - 1], t.l2e[m][kNS - 1]);
 #pragma unroll
@@ -382,7 +388,7 @@ __device__ __forceinline__ void rate_stage(const RateLane &t, float2 s, const fl
   }
   const float2 e = make_float2(ex2_approx(ntm.x), ex2_approx(ntm.y));
   float2 w = __fmul2_rn(__fmul2_rn(s, e), sinhc_half2<kForm == 0>(dl));
-  if (kForm == 2) {
+  if (kForm == 2 && sfu) {
     const float kLn2 = 0.69314718055994531f;
     const float2 ntl = __ffma2_rn(dl, both(0.5f), ntm);
     const float q0 = s.x * ex2_approx(ntl.x) * __fdividef(1.0f - ex2_approx(-dl.x), dl.x * kLn2);
@@ -398,11 +404,11 @@ __device__ __forceinline__ void rate_stage(const RateLane &t, float2 s, const fl
 }
 template <int f0, int f1, int f2, int f3>
 __device__ __forceinline__ void ray_stages(const RateLane &t, const float2 (&sp)[4], const float2 (&n)[3],
-                                           const float2 (&d)[3], float2 (&acc)[6]) {
+                                           const float2 (&d)[3], float2 (&acc)[6], int form = 5) {
   rate_stage<0, 2, f0>(t, sp[0], n, d, acc);
   rate_stage<1, 3, f1>(t, sp[1], n, d, acc);
-  rate_stage<2, 3, f2>(t, sp[2], n, d, acc);
-  rate_stage<3, 3, f3>(t, sp[3], n, d, acc);
+  rate_stage<2, 3, f2>(t, sp[2], n, d, acc, form >= 4);
+  rate_stage<3, 3, f3>(t, sp[3], n, d, acc, form == 5);
 }
 
 // The lane's partial sums of one ray: out[s] = (sum (sigma_s log2 e) w, sum
@@ -430,7 +436,7 @@ __device__ __forceinline__ void ray_bins(const RateLane &t, const RayRec *__rest
   if (form == 0) ray_stages<1, 0, 0, 0>(t, sp, n, d, acc);
   else if (form == 1) ray_stages<1, 1, 0, 0>(t, sp, n, d, acc);
   else if (form == 2) ray_stages<2, 1, 1, 1>(t, sp, n, d, acc);
-  else ray_stages<2, 2, 2, 2>(t, sp, n, d, acc);
+  else ray_stages<2, 2, 2, 2>(t, sp, n, d, acc, form);
 #pragma unroll
   for (int q = 0; q < 3; q++) out[q] = make_float2(acc[q].x + acc[q].y, acc[3 + q].x + acc[3 + q].y);
 }

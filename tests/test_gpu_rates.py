@@ -211,3 +211,33 @@ def test_exact_f64_odd_fields(cuda_ok, oracle, what):
     ok = np.isfinite(want)
     assert ok.all() == (what == "zeros")
     assert (np.abs(rates[ok] - want[ok]) <= F64_RTOL * np.abs(want[ok])).all()
+
+
+def test_thick_cells_pay_for_the_stages_that_need_it(cuda_ok):
+    """Cells of optical depth 7 need the costlier form of the cell factor in
+    the lower half of the bins only: measured 1.3 times the time of thin
+    cells, 1.6 times if all bins took it."""
+    import torch
+    from argot_b200 import workload as W
+    from argot_b200.pipeline import Problem
+    times = []
+    for depth in (0.5, 7.0):
+        wl = W.plain(64, 16, seed=1)
+        wl.dens = (wl.dens * np.float32(depth * 64 / 128)).astype(np.float32)
+        pb = Problem(wl)
+        g = pb.groups[0]
+        rays, tau = pb.alloc_group_buffers()
+        pb.emit(g, rays)
+        pb.march(g, rays, tau)
+        rates = torch.zeros(6 * pb.ncell, device="cuda")
+        t = []
+        for _ in range(12):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            pb.rates(g, rays, tau, rates)
+            b.record()
+            b.synchronize()
+            t.append(a.elapsed_time(b))
+        times.append(min(t))
+        pb.close()
+    assert times[1] < 1.45 * times[0], times
