@@ -237,6 +237,34 @@ __global__ void __launch_bounds__(32 * kSplitRateWarps, ARGOT_SPLIT_RATE_MIN_CTA
   }
 }
 
+// The same with a CTA per block, for a part of few blocks (as
+// k_rate_f32_cta, at the same line): one warp per block leaves most warps
+// without one and the others with a long chain.  The step with it, tiles of
+// one block: 8 problems of 16^3 cells / 4 sources in 4 parts 0.46 -> 0.15 ms, 8 of
+// 32^3 / 30 in 4 parts 3.25 -> 2.62 ms, 20^3 / 300 in one part 3.80 -> 1.15 ms.
+__global__ void __launch_bounds__(32 * kSplitRateWarps, ARGOT_SPLIT_RATE_MIN_CTAS)
+    k_batch_rates_cta(const BatchProb *__restrict__ probs, const BatchItem *__restrict__ items, uint32_t i0,
+                      uint32_t i1, uint32_t sub, uint32_t *__restrict__ next) {
+  __shared__ RateWarpSmem s_w[kSplitRateWarps];
+  __shared__ int s_t[kSplitRateWarps][32];
+  __shared__ uint32_t s_it;
+  RateLane tab;
+  load_rate_lane(threadIdx.x & 31, tab);
+  for (;;) {
+    if (threadIdx.x == 0) s_it = atomicAdd(next, 1u);
+    __syncthreads();
+    const uint32_t it = s_it;
+    __syncthreads();
+    if (it >= (i1 - i0) * sub) break;
+    const BatchItem wi = sub_item(items[i0 + it / sub], it % sub, sub);
+    const BatchProb &P = probs[wi.prob];
+    const GridDev g = P.g;
+    for (uint64_t b = wi.b0; b < wi.b1; b++)
+      rate_block_f32_cta<kSplitRateWarps>(g, P.raw, P.emit_pos, P.specn, P.total, tab, b, P.blk_off[b],
+                                          P.blk_off[b + 1], P.rays, P.nray, P.tau, P.rates6, s_w, s_t);
+  }
+}
+
 }  // namespace argot
 
 using namespace argot;
@@ -250,6 +278,7 @@ struct argot_b200_batch {
   BatchItem *items_dev = nullptr;
   size_t items_cap = 0;
   uint32_t nitems = 0;
+  std::vector<uint64_t> item_blk;  // blocks of the items before each, and of all
   uint32_t *next_dev = nullptr;
   int *err = nullptr;
   argot_b200_batch_config cfg{8, 0, 4, 0, 0, 8};
@@ -264,7 +293,7 @@ struct argot_b200_batch {
   cudaStream_t side_cap = nullptr;  // the rates' stream while capturing
   std::vector<cudaEvent_t> ev;      // fork, one per part, join
   uint32_t *counters = nullptr;     // two per part
-  int grid_march = 0, grid_rates = 0;
+  int grid_march = 0, grid_rates = 0, grid_rates_cta = 0;
 };
 
 namespace {
@@ -321,6 +350,9 @@ int ensure_split(argot_b200_batch *b) {
   b->grid_march = b->sms * (n > 0 ? n : 1);
   ARGOT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batch_rates, 32 * kSplitRateWarps, 0));
   b->grid_rates = b->sms * (n > 0 ? n : 1);
+  ARGOT_CUDA_TRY(
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batch_rates_cta, 32 * kSplitRateWarps, 0));
+  b->grid_rates_cta = b->sms * (n > 0 ? n : 1);
   return 0;
 }
 
@@ -360,6 +392,8 @@ int build_items(argot_b200_batch *b) {
   if (!items.empty())
     ARGOT_CUDA_TRY(cudaMemcpy(b->items_dev, items.data(), sizeof(BatchItem) * items.size(), cudaMemcpyHostToDevice));
   b->nitems = (uint32_t)items.size();
+  b->item_blk.assign(items.size() + 1, 0);
+  for (size_t i = 0; i < items.size(); i++) b->item_blk[i + 1] = b->item_blk[i] + (items[i].b1 - items[i].b0);
   const int occ = max_ctas_per_sm(b->cfg.warps_per_cta);
   if (occ <= 0) return ARGOT_B200_ECUDA;
   const int per_sm = b->cfg.ctas_per_sm > 0 ? std::min(b->cfg.ctas_per_sm, occ) : occ;
@@ -392,8 +426,15 @@ int launch_split(argot_b200_batch *b, unsigned long long *crossings, cudaStream_
     ARGOT_CUDA_TRY(cudaGetLastError());
     ARGOT_CUDA_TRY(cudaEventRecord(b->ev[1 + p], st));
     ARGOT_CUDA_TRY(cudaStreamWaitEvent(side, b->ev[1 + p], 0));
-    k_batch_rates<<<b->grid_rates, 32 * kSplitRateWarps, 0, side>>>(
-        b->probs_dev, b->items_dev, i0, i1, units(b->grid_rates * kSplitRateWarps), b->counters + 2 * p + 1);
+    const uint64_t nblk = b->item_blk[i1] - b->item_blk[i0], slots = (uint64_t)b->grid_rates * kSplitRateWarps;
+    if (nblk < kCtaBlocks * slots)  // (one unit per block)
+      k_batch_rates_cta<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(nblk, b->grid_rates_cta)),
+                          32 * kSplitRateWarps, 0, side>>>(b->probs_dev, b->items_dev, i0, i1,
+                                                           (uint32_t)b->cfg.blocks_per_item,
+                                                           b->counters + 2 * p + 1);
+    else
+      k_batch_rates<<<b->grid_rates, 32 * kSplitRateWarps, 0, side>>>(
+          b->probs_dev, b->items_dev, i0, i1, units(b->grid_rates * kSplitRateWarps), b->counters + 2 * p + 1);
     ARGOT_CUDA_TRY(cudaGetLastError());
   }
   ARGOT_CUDA_TRY(cudaEventRecord(b->ev[1 + parts], side));

@@ -119,26 +119,11 @@ __global__ void __launch_bounds__(32 * kF32Warps, ARGOT_RATE_MIN_CTAS)
   }
 }
 
-// The same with a CTA per block, for ranges of few blocks: the CTA's warps
-// take the block's chunks in turn, four at a time, then warps 0 to 2 add
-// them in order, two of the six rates each (the same sums, bit for bit).
+// The same with a CTA per block (rate_block_f32_cta), for ranges of few blocks.
 // Measured against one warp per block: 32^3 cells / 8 sources (1024 blocks of
 // 200 rays) 110 -> 88 us, 48^3 / 64 (3456 blocks of 1460) 1.54 -> 1.32 ms;
 // 64^3 / 16 (8192 of 420) 0.94 against 0.82 ms, the warps' waits outweighing
 // the better split: hence the line at two blocks per warp slot.
-struct CellSumPair {
-  float (*a)[32];
-  int lane, q0;
-  __device__ __forceinline__ void add(const float *v) {
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-      float s = a[q0 + i][lane], c = a[6 + q0 + i][lane];
-      kahan_add(s, c, v[q0 + i]);
-      a[q0 + i][lane] = s;
-      a[6 + q0 + i][lane] = c;
-    }
-  }
-};
 __global__ void __launch_bounds__(32 * kF32Warps, ARGOT_RATE_MIN_CTAS)
     k_rate_f32_cta(GridDev g, const float4 *__restrict__ raw, const float4 *__restrict__ emit_pos,
                    const float *__restrict__ specn, const double *__restrict__ total, uint64_t b0, uint64_t b1,
@@ -146,45 +131,17 @@ __global__ void __launch_bounds__(32 * kF32Warps, ARGOT_RATE_MIN_CTAS)
                    uint64_t nray, const float *__restrict__ tau, float *__restrict__ rates6, int *__restrict__ err) {
   __shared__ RateWarpSmem s_w[kF32Warps];
   __shared__ int s_t[kF32Warps][32];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const uint64_t ncell = (uint64_t)g.nx * g.ny * g.nz;
   RateLane tab;
-  load_rate_lane(lane, tab);
+  load_rate_lane(threadIdx.x & 31, tab);
   for (uint64_t b = b0 + blockIdx.x; b < b1; b += gridDim.x) {
     uint64_t r0, r1;
     if (!block_rays(blk_off, b, base, nray, &r0, &r1)) {
       if (threadIdx.x == 0) atomicExch(err, 1);
       continue;
     }
-    int ix, iy, iz, bix, biy, biz;
-    const bool own_valid = block_cell(g, b, lane, &ix, &iy, &iz);
-    block_cell(g, b, 0, &bix, &biy, &biz);
-    CellSumPair acc{s_w[0].acc, lane, 2 * wib};
-    if (wib < 3) {
-#pragma unroll
-      for (int i = 0; i < 2; i++) acc.a[acc.q0 + i][lane] = acc.a[6 + acc.q0 + i][lane] = 0.f;
-    }
-    for (uint64_t rs = r0; rs < r1; rs += 32 * kF32Warps) {
-      const uint64_t rc = rs + 32 * wib;
-      s_t[wib][lane] = rc < r1 ? rate_chunk<false>(g, raw, emit_pos, specn, total, tab, bix, biy, biz, rc, r1, rays,
-                                                   nray, tau, s_w[wib], lane, nullptr)
-                               : -1;
-      __syncthreads();
-      if (wib < 3) {
-        for (int v = 0; v < kF32Warps; v++)
-          add_chunk_in_order(acc, lane, s_t[v][lane], s_w[v].c.out, s_w[wib].cnt, s_w[wib].src);
-      }
-      __syncthreads();
-    }
-    if (wib < 3 && own_valid) {
-      const uint64_t own = cell_index(g, ix, iy, iz);
-#pragma unroll
-      for (int i = 0; i < 2; i++) rates6[(acc.q0 + i) * ncell + own] = acc.a[acc.q0 + i][lane];
-    }
+    rate_block_f32_cta<kF32Warps>(g, raw, emit_pos, specn, total, tab, b, r0, r1, rays, nray, tau, rates6, s_w, s_t);
   }
 }
-constexpr uint64_t kCtaBlocks = 2;  // blocks per warp slot below which a block takes a CTA
-static_assert(kF32Warps >= 3, "three warps add a block's rates");
 
 // The FP32 rates of blocks [b0, b1) where the rays flagged in pred (7
 // planes: six contributions and a flag, see rate_block_f32) keep their

@@ -649,4 +649,60 @@ __device__ __forceinline__ void rate_block_f32(const GridDev &g, const float4 *_
   }
 }
 
+// The same by a CTA of kWarps warps: they take the block's chunks in turn,
+// kWarps at a time, then warps 0 to 2 add them in order, two of the six rates
+// each (the same sums, bit for bit).  Starts and ends with its shared memory
+// free (a barrier after the last use, but for the sums of the warps' own).
+struct CellSumPair {
+  float (*a)[32];
+  int lane, q0;
+  __device__ __forceinline__ void add(const float *v) {
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      float s = a[q0 + i][lane], c = a[6 + q0 + i][lane];
+      kahan_add(s, c, v[q0 + i]);
+      a[q0 + i][lane] = s;
+      a[6 + q0 + i][lane] = c;
+    }
+  }
+};
+constexpr uint64_t kCtaBlocks = 2;  // blocks per warp slot below which a block takes a CTA
+template <int kWarps>
+__device__ __forceinline__ void rate_block_f32_cta(const GridDev &g, const float4 *__restrict__ raw,
+                                                   const float4 *__restrict__ emit_pos,
+                                                   const float *__restrict__ specn, const double *__restrict__ total,
+                                                   const RateLane &tab, uint64_t b, uint64_t r0, uint64_t r1,
+                                                   const uint32_t *__restrict__ rays, uint64_t nray,
+                                                   const float *__restrict__ tau, float *__restrict__ rates6,
+                                                   RateWarpSmem (&S)[kWarps], int (&t)[kWarps][32]) {
+  static_assert(kWarps >= 3, "three warps add a block's rates");
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const uint64_t ncell = (uint64_t)g.nx * g.ny * g.nz;
+  int ix, iy, iz, bix, biy, biz;
+  const bool own_valid = block_cell(g, b, lane, &ix, &iy, &iz);
+  block_cell(g, b, 0, &bix, &biy, &biz);
+  CellSumPair acc{S[0].acc, lane, 2 * wib};
+  if (wib < 3) {
+#pragma unroll
+    for (int i = 0; i < 2; i++) acc.a[acc.q0 + i][lane] = acc.a[6 + acc.q0 + i][lane] = 0.f;
+  }
+  for (uint64_t rs = r0; rs < r1; rs += 32 * kWarps) {
+    const uint64_t rc = rs + 32 * wib;
+    t[wib][lane] = rc < r1 ? rate_chunk<false>(g, raw, emit_pos, specn, total, tab, bix, biy, biz, rc, r1, rays, nray,
+                                               tau, S[wib], lane, nullptr)
+                           : -1;
+    __syncthreads();
+    if (wib < 3) {
+      for (int v = 0; v < kWarps; v++)
+        add_chunk_in_order(acc, lane, t[v][lane], S[v].c.out, S[wib].cnt, S[wib].src);
+    }
+    __syncthreads();
+  }
+  if (wib < 3 && own_valid) {
+    const uint64_t own = cell_index(g, ix, iy, iz);
+#pragma unroll
+    for (int i = 0; i < 2; i++) rates6[(acc.q0 + i) * ncell + own] = acc.a[acc.q0 + i][lane];
+  }
+}
+
 }  // namespace argot

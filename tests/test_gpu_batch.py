@@ -101,3 +101,21 @@ def test_batch_autotuner(batch, solo):
     _clear(batch)
     batch.graph_launch()
     _check(batch, solo)
+
+
+@pytest.mark.parametrize("blocks_per_item", [1, 100])
+def test_batch_parts_of_few_and_many_blocks(cuda_ok, blocks_per_item):
+    """A part of many blocks takes a warp per block, one of few a CTA: the
+    same rates as the problems alone, also where a tile ends short."""
+    import torch
+    from argot_b200 import workload as W
+    from argot_b200.batch import Batch
+    b = Batch([W.tiny(48, 3, seed=1), W.tiny(50, 5, seed=2)])  # 3456 and 4225 blocks
+    want = [pb.run().clone() for pb in b.problems]
+    for parts in (1, 2, 13):
+        b.configure(mode=1, parts=parts, blocks_per_item=blocks_per_item)
+        _clear(b)
+        b.run()
+        assert all(torch.equal(r, w) for r, w in zip(b.rates, want))
+    b.check_device_error()
+    b.close()
