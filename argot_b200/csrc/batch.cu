@@ -28,6 +28,7 @@
 #include <mutex>
 #include <new>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include "march.cuh"
@@ -55,20 +56,29 @@ struct BatchItem {
   uint32_t prob, b0, b1, pad;
 };
 
-// Launch shape: kWarps warps per CTA and at least ARGOT_BATCH_MIN_WARPS / kWarps
-// CTAs resident per SM (which caps the registers per thread).  Measured on
-// B200 (8 problems of 32^3 to 96^3 cells): 24 warps per SM (80 registers)
-// 78.4 ms, 16 warps 81.0 ms, 32 warps (64 registers, spilling the rates'
-// tables) 89.5 ms.
-#ifndef ARGOT_BATCH_MIN_WARPS
-#define ARGOT_BATCH_MIN_WARPS 24
-#endif
-template <int kWarps>
-__global__ void __launch_bounds__(32 * kWarps, ARGOT_BATCH_MIN_WARPS / kWarps)
+// Launch shape: CTAs of kWarps warps, as many per SM as make up the warps
+// below (which caps the registers per thread).  The march wants warps, the
+// rates registers for the lane's cross sections; with those in shared memory
+// both have them, and a batch that fills the GPU runs so.  One whose tiles
+// fit one fill of the other launch keeps them in registers.  Measured on
+// B200, 48 problems of 32^3 to 128^3 cells and 8 of 32^3 to 96^3, CTAs of 8
+// warps: shared, 32 warps per SM (64 registers) 1.55 s and 77.0 ms, 24 warps 1.75 s
+// and 81.8 ms; registers, 24 warps (80 registers) 1.74 s and 78.4 ms, 16 warps
+// 1.93 s and 81.0 ms, 32 warps (spilling them) 1.87 s and 88.9 ms.  Of one fill
+// or less, shared and registers: 64^3 cells / 100 sources 10.9 and 10.2 ms, 20^3 /
+// 300 13.9 and 13.2 ms, 8 problems of 16^3 / 4 0.42 and 0.41 ms.
+constexpr int kSharedWarps = 32, kRegisterWarps = 24;
+template <int kWarps, bool kShared>
+__global__ void __launch_bounds__(32 * kWarps, (kShared ? kSharedWarps : kRegisterWarps) / kWarps)
     k_batch(const BatchProb *__restrict__ probs, const BatchItem *__restrict__ items, uint32_t nitems,
             uint32_t *__restrict__ next, unsigned long long *__restrict__ crossings, int *__restrict__ err) {
   __shared__ RateChunk s_c[kWarps];
   __shared__ int s_cnt[kWarps][32], s_src[kWarps][32];
+  __shared__ std::conditional_t<kShared, RateTab, int> s_tab;  // (unused in registers)
+  if constexpr (kShared) {
+    load_rate_tab(s_tab);
+    __syncthreads();
+  }
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   unsigned long long steps_total = 0;
   bool bad = false;
@@ -121,15 +131,17 @@ __global__ void __launch_bounds__(32 * kWarps, ARGOT_BATCH_MIN_WARPS / kWarps)
                                              tt.heii, rw, __ldg(total + e));
           s_c[wib].rec[lane] = ray_rec(p, (int)e);
 #pragma unroll
-          for (int s = 0; s < 3; s++) s_c[wib].p[lane][s] = p.P[s];
+          for (int s = 0; s < 3; s++) s_c[wib].out[lane][s] = p.P[s];
         }
         __syncwarp();
-        {
-          // the lane's cross sections, read again for every chunk so that
-          // the march does not carry them
+        const int nk = (int)min((uint64_t)32, r1 - rc);
+        if constexpr (kShared) {
+          chunk_rates(s_c[wib], RateShared{&s_tab, lane}, specn, nullptr, nk, lane);
+        } else {
+          // read again for every chunk so that the march does not carry them
           RateLane tab;
           load_rate_lane(lane, tab);
-          chunk_rates(s_c[wib], tab, specn, nullptr, (int)min((uint64_t)32, r1 - rc), lane);
+          chunk_rates(s_c[wib], tab, specn, nullptr, nk, lane);
         }
         __syncwarp();
         add_chunk_in_order(acc, lane, t, s_c[wib].out, s_cnt[wib], s_src[wib]);
@@ -283,6 +295,7 @@ struct argot_b200_batch {
   int *err = nullptr;
   argot_b200_batch_config cfg{8, 0, 4, 0, 0, 8};
   int grid = 0;
+  bool shared = true;  // the fused kernel's table in shared memory
   cudaStream_t cap = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -305,10 +318,16 @@ void drop_graph(argot_b200_batch *b) {
   b->graph = nullptr;
 }
 
-int max_ctas_per_sm(int warps) {
+// The fused kernel for CTAs of `warps` warps.
+using FusedKernel = void (*)(const BatchProb *, const BatchItem *, uint32_t, uint32_t *, unsigned long long *, int *);
+FusedKernel fused_kernel(int warps, bool shared) {
+  if (warps == 4) return shared ? k_batch<4, true> : k_batch<4, false>;
+  return shared ? k_batch<8, true> : k_batch<8, false>;
+}
+
+int max_ctas_per_sm(int warps, bool shared = true) {
   int n = 0;
-  cudaError_t e = warps == 4 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batch<4>, 128, 0)
-                             : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batch<8>, 256, 0);
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fused_kernel(warps, shared), 32 * warps, 0);
   return e == cudaSuccess ? n : 0;
 }
 
@@ -394,7 +413,8 @@ int build_items(argot_b200_batch *b) {
   b->nitems = (uint32_t)items.size();
   b->item_blk.assign(items.size() + 1, 0);
   for (size_t i = 0; i < items.size(); i++) b->item_blk[i + 1] = b->item_blk[i] + (items[i].b1 - items[i].b0);
-  const int occ = max_ctas_per_sm(b->cfg.warps_per_cta);
+  b->shared = b->nitems > (uint32_t)(kRegisterWarps * b->sms);
+  const int occ = max_ctas_per_sm(b->cfg.warps_per_cta, b->shared);
   if (occ <= 0) return ARGOT_B200_ECUDA;
   const int per_sm = b->cfg.ctas_per_sm > 0 ? std::min(b->cfg.ctas_per_sm, occ) : occ;
   const uint64_t warps_needed = std::max<uint64_t>(1, b->nitems);
@@ -449,10 +469,8 @@ int launch(argot_b200_batch *b, unsigned long long *crossings, cudaStream_t st, 
     return launch_split(b, crossings, st, capturing ? b->side_cap : b->side);
   }
   ARGOT_CUDA_TRY(cudaMemsetAsync(b->next_dev, 0, sizeof(uint32_t), st));
-  if (b->cfg.warps_per_cta == 4)
-    k_batch<4><<<b->grid, 128, 0, st>>>(b->probs_dev, b->items_dev, b->nitems, b->next_dev, crossings, b->err);
-  else
-    k_batch<8><<<b->grid, 256, 0, st>>>(b->probs_dev, b->items_dev, b->nitems, b->next_dev, crossings, b->err);
+  fused_kernel(b->cfg.warps_per_cta, b->shared)<<<b->grid, 32 * b->cfg.warps_per_cta, 0, st>>>(
+      b->probs_dev, b->items_dev, b->nitems, b->next_dev, crossings, b->err);
   ARGOT_CUDA_TRY(cudaGetLastError());
   return 0;
 }

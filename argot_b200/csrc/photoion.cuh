@@ -284,18 +284,30 @@ __device__ __forceinline__ RayParams ray_params_f32(const GridDev &g, int gix, i
 // against 130 and 23 now.  256^3 cells, 1024 clustered sources, 2.17e9 rays:
 // 0.524 s before, 0.471 s now.  Two rays at a time per warp (for more
 // independent chains): 0.461 s alone, the step with the march no faster.
+// (RateShared reads them from a copy in shared memory instead, for a kernel
+// that needs its registers.)
 struct RateLane {
-  float2 l2e[4][3];  // sigma_s log2(e) of the lane's two bins of each stage
-  float2 h[4][3];    // sigma_s log2(e) (nu - nu_s)^+
+  float2 v[kStages][6];
+  __device__ __forceinline__ float2 l2e(int m, int s) const { return v[m][s]; }    // sigma_s log2(e)
+  __device__ __forceinline__ float2 h(int m, int s) const { return v[m][3 + s]; }  // sigma_s log2(e) (nu - nu_s)^+
 };
 __device__ __forceinline__ void load_rate_lane(int lane, RateLane &r) {
 #pragma unroll
   for (int m = 0; m < kStages; m++)
 #pragma unroll
-    for (int s = 0; s < 3; s++) {
-      r.l2e[m][s] = __ldg(&d_rate_tab.v[m][s][lane]);
-      r.h[m][s] = __ldg(&d_rate_tab.v[m][3 + s][lane]);
-    }
+    for (int s = 0; s < 6; s++) r.v[m][s] = __ldg(&d_rate_tab.v[m][s][lane]);
+}
+struct RateShared {
+  const RateTab *tab;
+  int lane;
+  __device__ __forceinline__ float2 l2e(int m, int s) const { return tab->v[m][s][lane]; }
+  __device__ __forceinline__ float2 h(int m, int s) const { return tab->v[m][3 + s][lane]; }
+};
+// Fills a CTA's copy (all threads; the caller synchronises).
+__device__ __forceinline__ void load_rate_tab(RateTab &t) {
+  const float2 *from = &d_rate_tab.v[0][0][0];
+  float2 *to = &t.v[0][0][0];
+  for (int i = threadIdx.x; i < kStages * 6 * 32; i += blockDim.x) to[i] = __ldg(from + i);
 }
 
 // The photon-conserving cell factor phi(x) = (1 - e^-x)/x (x the cell's
@@ -376,15 +388,15 @@ __device__ __forceinline__ RayRec ray_rec(const RayParams &p, int e) {
 // sections; kForm as in ray_form.  ntm = -(tau + x / 2) log2(e), w = s 2^ntm
 // sinh(x/2)/(x/2) or, with kForm 2, sfu and x >= kPhiXMax, s 2^(ntm + dl/2)
 // (1 - 2^-dl) / x.
-template <int m, int kNS, int kForm>
-__device__ __forceinline__ void rate_stage(const RateLane &t, float2 s, const float2 (&n)[3], const float2 (&d)[3],
+template <int m, int kNS, int kForm, class Tab>
+__device__ __forceinline__ void rate_stage(const Tab &t, float2 s, const float2 (&n)[3], const float2 (&d)[3],
                                            float2 (&acc)[6], bool sfu = true) {
-  float2 ntm = __fmul2_rn(n[kNS - 1], t.l2e[m][kNS - 1]);
-  float2 dl = __fmul2_rn(d[kNS - 1], t.l2e[m][kNS - 1]);
+  float2 ntm = __fmul2_rn(n[kNS - 1], t.l2e(m, kNS - 1));
+  float2 dl = __fmul2_rn(d[kNS - 1], t.l2e(m, kNS - 1));
 #pragma unroll
   for (int q = kNS - 2; q >= 0; q--) {
-    ntm = __ffma2_rn(n[q], t.l2e[m][q], ntm);
-    dl = __ffma2_rn(d[q], t.l2e[m][q], dl);
+    ntm = __ffma2_rn(n[q], t.l2e(m, q), ntm);
+    dl = __ffma2_rn(d[q], t.l2e(m, q), dl);
   }
   const float2 e = make_float2(ex2_approx(ntm.x), ex2_approx(ntm.y));
   float2 w = __fmul2_rn(__fmul2_rn(s, e), sinhc_half2<kForm == 0>(dl));
@@ -398,12 +410,12 @@ __device__ __forceinline__ void rate_stage(const RateLane &t, float2 s, const fl
   }
 #pragma unroll
   for (int q = 0; q < kNS; q++) {
-    acc[q] = __ffma2_rn(t.l2e[m][q], w, acc[q]);
-    acc[3 + q] = __ffma2_rn(t.h[m][q], w, acc[3 + q]);
+    acc[q] = __ffma2_rn(t.l2e(m, q), w, acc[q]);
+    acc[3 + q] = __ffma2_rn(t.h(m, q), w, acc[3 + q]);
   }
 }
-template <int f0, int f1, int f2, int f3>
-__device__ __forceinline__ void ray_stages(const RateLane &t, const float2 (&sp)[4], const float2 (&n)[3],
+template <int f0, int f1, int f2, int f3, class Tab>
+__device__ __forceinline__ void ray_stages(const Tab &t, const float2 (&sp)[4], const float2 (&n)[3],
                                            const float2 (&d)[3], float2 (&acc)[6], int form = 5) {
   rate_stage<0, 2, f0>(t, sp[0], n, d, acc);
   rate_stage<1, 3, f1>(t, sp[1], n, d, acc);
@@ -415,7 +427,8 @@ __device__ __forceinline__ void ray_stages(const RateLane &t, const float2 (&sp)
 // (sigma_s log2 e) (nu - nu_s)^+ w) over its bins, w = s_nu e^-tau phi(x).
 // sp: the lane's spectrum of emitter `cur`, read again when the ray's
 // emitter is another one (a block's rays come emitter by emitter).
-__device__ __forceinline__ void ray_bins(const RateLane &t, const RayRec *__restrict__ rec,
+template <class Tab>
+__device__ __forceinline__ void ray_bins(const Tab &t, const RayRec *__restrict__ rec,
                                          const float *__restrict__ specn, int lane, int &cur, float2 (&sp)[4],
                                          float2 (&out)[3]) {
   const float4 ra = *reinterpret_cast<const float4 *>(rec->n), rb = *reinterpret_cast<const float4 *>(rec->d);
@@ -447,18 +460,18 @@ constexpr int kRedRow = 34;  // float2 per row: 16-byte reads of 8 rows fall on 
 struct RateChunk {
   RayRec rec[32];
   float2 red[3 * kRoundRays][kRedRow];  // a round's lane sums, row 3 k + s: ray k, species s
-  float p[32][3];    // prefactors P_s
-  float out[32][6];  // per-ray rates
+  float out[32][6];  // prefactors P_s, then the rays' rates
 };
 
-// The rates of nq rays of a chunk (ray i is entry q[i], or i without q):
-// S.out[ray] = Gamma_s = P_s ln2 a_s, Heat_s = P_s ln2 b_s h nu_L.  All lanes
+// The rates of nq rays of a chunk (ray i is entry q[i], or i without q), S.out
+// holding their prefactors: S.out[ray] = Gamma_s = P_s ln2 a_s, Heat_s = P_s ln2 b_s h nu_L.  All lanes
 // of the warp take part; the caller synchronises the warp before and after.
 // Rounds of kRoundRays rays: every lane leaves its three pairs of sums per
 // ray in shared memory, then lane r and lane r + 16 add the lanes 0..15 and
 // 16..31 of row r (a butterfly over the warp takes 60 instructions per ray,
 // a recursive halving 25, this 10).
-__device__ __forceinline__ void chunk_rates(RateChunk &S, const RateLane &t, const float *__restrict__ specn,
+template <class Tab>
+__device__ __forceinline__ void chunk_rates(RateChunk &S, const Tab &t, const float *__restrict__ specn,
                                             const int *q, int nq, int lane) {
   const float kLn2 = 0.69314718055994531f;
   const int row = lane & 15, kr = row / 3, s = row - 3 * kr;
@@ -491,7 +504,7 @@ __device__ __forceinline__ void chunk_rates(RateChunk &S, const RateLane &t, con
     sum.y += __shfl_xor_sync(0xffffffffu, sum.y, 16);
     if (kr < nr && lane < 16) {
       const int ray = q ? q[i + kr] : i + kr;
-      const float P = S.p[ray][s];
+      const float P = S.out[ray][s];
       S.out[ray][s] = P * (kLn2 * sum.x);
       S.out[ray][3 + s] = P * (kLn2 * sum.y) * kHNuLf;
     }
@@ -597,7 +610,7 @@ __device__ __forceinline__ int rate_chunk(const GridDev &g, const float4 *__rest
                                          __ldg(tau + nray + r), __ldg(tau + 2 * nray + r), rw, __ldg(total + e));
       S.c.rec[lane] = ray_rec(p, (int)e);
 #pragma unroll
-      for (int s = 0; s < 3; s++) S.c.p[lane][s] = p.P[s];
+      for (int s = 0; s < 3; s++) S.c.out[lane][s] = p.P[s];
     }
   }
   int nq = (int)min((uint64_t)32, r1 - rc);
