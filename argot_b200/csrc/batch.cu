@@ -249,9 +249,9 @@ __global__ void __launch_bounds__(32 * kSplitRateWarps, ARGOT_SPLIT_RATE_MIN_CTA
   }
 }
 
-// The same with a CTA per block, for a part of few blocks (as
-// k_rate_f32_cta, at the same line): one warp per block leaves most warps
-// without one and the others with a long chain.  The step with it, tiles of
+// The same with a CTA per block, for a part of few blocks (cta_per_block):
+// one warp per block leaves most warps without one and the others with a long
+// chain.  The step with it, tiles of
 // one block: 8 problems of 16^3 cells / 4 sources in 4 parts 0.46 -> 0.15 ms, 8 of
 // 32^3 / 30 in 4 parts 3.25 -> 2.62 ms, 20^3 / 300 in one part 3.80 -> 1.15 ms.
 __global__ void __launch_bounds__(32 * kSplitRateWarps, ARGOT_SPLIT_RATE_MIN_CTAS)
@@ -290,7 +290,7 @@ struct argot_b200_batch {
   BatchItem *items_dev = nullptr;
   size_t items_cap = 0;
   uint32_t nitems = 0;
-  std::vector<uint64_t> item_blk;  // blocks of the items before each, and of all
+  std::vector<uint64_t> item_blk, item_ray;  // blocks and rays of the items before each, and of all
   uint32_t *next_dev = nullptr;
   int *err = nullptr;
   argot_b200_batch_config cfg{8, 0, 4, 0, 0, 8};
@@ -412,7 +412,12 @@ int build_items(argot_b200_batch *b) {
     ARGOT_CUDA_TRY(cudaMemcpy(b->items_dev, items.data(), sizeof(BatchItem) * items.size(), cudaMemcpyHostToDevice));
   b->nitems = (uint32_t)items.size();
   b->item_blk.assign(items.size() + 1, 0);
-  for (size_t i = 0; i < items.size(); i++) b->item_blk[i + 1] = b->item_blk[i] + (items[i].b1 - items[i].b0);
+  b->item_ray.assign(items.size() + 1, 0);
+  for (size_t i = 0; i < items.size(); i++) {
+    const std::vector<uint64_t> &off = b->blk_off[items[i].prob];
+    b->item_blk[i + 1] = b->item_blk[i] + (items[i].b1 - items[i].b0);
+    b->item_ray[i + 1] = b->item_ray[i] + (off[items[i].b1] - off[items[i].b0]);
+  }
   b->shared = b->nitems > (uint32_t)(kRegisterWarps * b->sms);
   const int occ = max_ctas_per_sm(b->cfg.warps_per_cta, b->shared);
   if (occ <= 0) return ARGOT_B200_ECUDA;
@@ -446,9 +451,9 @@ int launch_split(argot_b200_batch *b, unsigned long long *crossings, cudaStream_
     ARGOT_CUDA_TRY(cudaGetLastError());
     ARGOT_CUDA_TRY(cudaEventRecord(b->ev[1 + p], st));
     ARGOT_CUDA_TRY(cudaStreamWaitEvent(side, b->ev[1 + p], 0));
-    const uint64_t nblk = b->item_blk[i1] - b->item_blk[i0], slots = (uint64_t)b->grid_rates * kSplitRateWarps;
-    if (nblk < kCtaBlocks * slots)  // (one unit per block)
-      k_batch_rates_cta<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(nblk, b->grid_rates_cta)),
+    const uint64_t nblk = b->item_blk[i1] - b->item_blk[i0];
+    if (cta_per_block(nblk, b->item_ray[i1] - b->item_ray[i0], (uint64_t)b->grid_rates_cta, kSplitRateWarps))
+      k_batch_rates_cta<<<(unsigned)std::min<uint64_t>(nblk, b->grid_rates_cta),  // (one unit per block)
                           32 * kSplitRateWarps, 0, side>>>(b->probs_dev, b->items_dev, i0, i1,
                                                            (uint32_t)b->cfg.blocks_per_item,
                                                            b->counters + 2 * p + 1);

@@ -120,10 +120,7 @@ __global__ void __launch_bounds__(32 * kF32Warps, ARGOT_RATE_MIN_CTAS)
 }
 
 // The same with a CTA per block (rate_block_f32_cta), for ranges of few blocks.
-// Measured against one warp per block: 32^3 cells / 8 sources (1024 blocks of
-// 200 rays) 110 -> 88 us, 48^3 / 64 (3456 blocks of 1460) 1.54 -> 1.32 ms;
-// 64^3 / 16 (8192 of 420) 0.94 against 0.82 ms, the warps' waits outweighing
-// the better split: hence the line at two blocks per warp slot.
+// When that pays: cta_per_block.
 __global__ void __launch_bounds__(32 * kF32Warps, ARGOT_RATE_MIN_CTAS)
     k_rate_f32_cta(GridDev g, const float4 *__restrict__ raw, const float4 *__restrict__ emit_pos,
                    const float *__restrict__ specn, const double *__restrict__ total, uint64_t b0, uint64_t b1,
@@ -202,7 +199,7 @@ extern "C" int argot_b200_photoion_rays(const argot_b200_grid *gp, const void *p
   if (mode == ARGOT_B200_RATE_EXACT_F64)
     k_rate_blocks<<<blocks, threads, 0, st>>>(g, raw, t->emit_pos, t->emit_spec64, b0, b1, blk_off, base, rays,
                                               nray, tau, rates6, err);
-  else if (b1 - b0 < (uint64_t)sms * ARGOT_RATE_MIN_CTAS * kF32Warps * kCtaBlocks)
+  else if (cta_per_block(b1 - b0, nray, (uint64_t)sms * ARGOT_RATE_MIN_CTAS, kF32Warps))
     k_rate_f32_cta<<<(unsigned)std::min<uint64_t>(b1 - b0, 16ull * sms), 32 * kF32Warps, 0, st>>>(
         g, raw, t->emit_pos, t->emit_specn, t->emit_total, b0, b1, blk_off, base, rays, nray, tau, rates6, err);
   else

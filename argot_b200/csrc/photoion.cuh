@@ -679,7 +679,25 @@ struct CellSumPair {
     }
   }
 };
-constexpr uint64_t kCtaBlocks = 2;  // blocks per warp slot below which a block takes a CTA
+// Whether nblk blocks with nray rays take a CTA each rather than a warp, on a
+// GPU that holds `ctas` CTAs of `warps` warps: when the fills of the GPU times
+// the rounds of chunks in each are fewer.  Measured, CTA and warp: 32^3 cells /
+// 8 sources (1024 blocks of 7 chunks) 88 and 110 us, 24^3 / 2 (432 of 2) 19 and
+// 27, 32^3 / 5 (1024 of 5) 67 and 72, 48^3 / 64 (3456 of 46) 1.32 and 1.54 ms; but
+// 32^3 / 1 (1024 of 1) 27 and 19 us, 52^3 / 1 (4394 of 1) 88 and 43, 36^3 / 5 (1458 of
+// 5) 90 and 85.  With long blocks the CTAs also even out their differences, an
+// eighth: the step of 8 batched problems of 32^3 / 30 in 4 parts (2048 blocks of
+// about 19) 2.64 and 3.00 ms.  From two blocks per warp slot on the warps' waits
+// for one another outweigh the better split: 64^3 / 16 (8192 of 14) 0.94 and
+// 0.82 ms.
+static inline bool cta_per_block(uint64_t nblk, uint64_t nray, uint64_t ctas, uint64_t warps) {
+  const auto ceil_div = [](uint64_t a, uint64_t b) { return (a + b - 1) / b; };
+  if (nblk == 0 || nblk >= 2 * ctas * warps) return false;
+  const uint64_t chunks = ceil_div(nray, 32 * nblk);
+  const uint64_t by_cta = ceil_div(nblk, ctas) * ceil_div(chunks, warps);
+  const uint64_t by_warp = ceil_div(nblk, ctas * warps) * chunks;
+  return 8 * by_cta < (chunks > warps ? 9 : 8) * by_warp;
+}
 template <int kWarps>
 __device__ __forceinline__ void rate_block_f32_cta(const GridDev &g, const float4 *__restrict__ raw,
                                                    const float4 *__restrict__ emit_pos,
