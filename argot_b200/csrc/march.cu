@@ -152,9 +152,13 @@ __global__ void __launch_bounds__(256) k_walk(GridDev g, const DevNode *__restri
 // Launch shape: 64 warps per SM (32 registers) in CTAs of 16 warps.  A range
 // of few blocks is cut finer: each block's chunks of 32 rays into segments,
 // one warp each, until there are kMarchItems items per warp slot (32^3 cells
-// / 8 sources: 78 -> 41 us, 64^3 / 16: 0.49 -> 0.45 ms; more items per slot
-// on larger meshes: no change), in CTAs of 8 warps where those would leave
-// warp slots empty.  What lives across a ray's walk is kept out of
+// / 8 sources: 78 -> 34 us), in CTAs of 8 warps where those would leave warp
+// slots empty.  Fewer items leave a last fill that is nearly empty, more cost
+// the blocks' starts again (one item per block, 2, 4, 6 and 8 per slot: 64^3 /
+// 16 471, 442, 434, 422 and 466 us, 100^3 / 100 8.89, 9.19, 8.58, 8.58 and
+// 8.86 ms).  A range that fits one fill runs all at once in any order, and
+// its blocks are taken as they are (the tiles' divisions are 1 us of 24^3 / 1's
+// 17; 64^3 / 16 in order 408 us).  What lives across a ray's walk is kept out of
 // registers: the Kahan columns in per-thread shared-memory slots, the
 // block's state (item, ray count, packed coordinates, first ray; the same
 // for the warp's lanes) in per-warp shared memory, read back after each ray.
@@ -162,7 +166,7 @@ __global__ void __launch_bounds__(256) k_walk(GridDev g, const DevNode *__restri
 // bounding box), so rays start at their emitter and the launch contains no
 // call.
 constexpr int kMarchWide = 512, kMarchNarrow = 256;
-constexpr uint64_t kMarchItems = 2;
+constexpr uint64_t kMarchItems = 6;
 
 // One level of a tiled enumeration of nx * ny * nz blocks (tiles of tx * ty *
 // tz, those at the high ends clipped; tiles in (x, y, z) order with z
@@ -213,7 +217,7 @@ template <int kPrec, bool kInside, int kThreads>
 __global__ void __launch_bounds__(kThreads, 2048 / kThreads) k_march_rays(GridDev g, const float4 *__restrict__ cells,
                                                     const float4 *__restrict__ emit_pos, uint32_t b0,
                                                     uint32_t b1, const uint64_t *__restrict__ blk_off,
-                                                    uint32_t nseg, uint64_t base,
+                                                    uint32_t nseg, bool tiled, uint64_t base,
                                                     const uint32_t *__restrict__ rays, uint64_t nray,
                                                     float *__restrict__ tau,
                                                     unsigned long long *__restrict__ crossings,
@@ -237,7 +241,7 @@ __global__ void __launch_bounds__(kThreads, 2048 / kThreads) k_march_rays(GridDe
     const uint32_t cw = it / W, grp = cw / nseg, sg = cw - grp * nseg;
     const uint32_t rank = grp * W + (it - cw * W);
     if (rank >= b1 - b0) continue;
-    const uint32_t b = block_of_item((uint32_t)g.nby, (uint32_t)g.nbz, b0 + rank, b0, b1);
+    const uint32_t b = tiled ? block_of_item((uint32_t)g.nby, (uint32_t)g.nbz, b0 + rank, b0, b1) : b0 + rank;
     uint64_t r0, r1;
     if (!block_rays(blk_off, b, base, nray, &r0, &r1)) { bad = true; continue; }
     if (nseg > 1) {  // the segment's share of the block's chunks of 32 rays
@@ -518,7 +522,7 @@ int argot_b200_march_rays(const argot_b200_grid *gp, const void *packed, const a
 #define ARGOT_MARCH_LAUNCH(P, I)                                                            \
   (wide ? k_march_rays<P, I, kMarchWide> : k_march_rays<P, I, kMarchNarrow>)                \
       <<<blocks, threads, 0, st>>>(g, cells, t->emit_pos, (uint32_t)b0, (uint32_t)b1,       \
-                                   blk_off, (uint32_t)nseg, base, rays, nray, tau, crossings, err)
+                                   blk_off, (uint32_t)nseg, nblk > slots, base, rays, nray, tau, crossings, err)
   if (prec == ARGOT_B200_PRECISION_REFERENCE) {
     if (inside) ARGOT_MARCH_LAUNCH(ARGOT_B200_PRECISION_REFERENCE, true);
     else ARGOT_MARCH_LAUNCH(ARGOT_B200_PRECISION_REFERENCE, false);

@@ -288,3 +288,32 @@ def test_block_order_covers_every_range(cuda_ok, edge, nsrc):
             pb.march(RayGroup(b0, b1, lo, n), rays[lo:], part, prec)
             assert torch.equal(part.view(3, n), whole[:, lo:hi])
     pb.check_device_error()
+
+
+@pytest.mark.parametrize("edge,nsrc", [(9, 90), (20, 60), (33, 40), (48, 3)])
+def test_crossings_of_segmented_blocks(cuda_ok, edge, nsrc):
+    """A range of few blocks is marched in segments of each block's rays: it
+    counts the crossings that the blocks as a whole count (the fused batch),
+    in one range and in slabs."""
+    import torch
+    from argot_b200 import _lib as L, workload as W
+    from argot_b200.batch import Batch
+    from argot_b200.pipeline import RayGroup
+    b = Batch([W.tiny(edge, nsrc, seed=edge)])
+    b.configure(mode=0)
+    cnt = torch.zeros(3, dtype=torch.int64, device="cuda")
+    b.run(cnt[:1])
+    pb = b.problems[0]
+    g = pb.groups[0]
+    rays, tau = pb.alloc_group_buffers()
+    pb.emit(g, rays)
+    pb.march(g, rays, tau, L.PRECISION_KAHAN, cnt[1:2])
+    slab, off = ((edge + 3) // 4) ** 2, pb.blk_off_host
+    for b0 in range(0, pb.nblocks, slab):
+        b1 = min(b0 + slab, pb.nblocks)
+        lo, n = int(off[b0]), int(off[b1] - off[b0])
+        pb.march(RayGroup(b0, b1, lo, n), rays[lo:], tau, L.PRECISION_KAHAN, cnt[2:])
+    pb.check_device_error()
+    n = cnt.tolist()
+    assert n[0] > pb.nray and n[0] == n[1] == n[2]
+    b.close()
