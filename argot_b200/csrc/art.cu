@@ -638,10 +638,38 @@ __global__ void __launch_bounds__(256) k_art_gather(uint64_t n, int ny, int nz, 
   }
 }
 
-// The six rates of a cell from the swept angles' sums m_i = sum over angles
-// of (sum of I (1 - e^-tau)) d / L, id = 1 / d [cm^-1] and the number of those angles
-// (calc_GH_tot.c:178-247), plus the general march's totals gh6, over all
-// angles.  tot6: gh6 (kGeneral) or the earlier groups' totals.
+// The six terms of a cell from the sums m_i = sum over nswept swept angles of
+// (sum of I (1 - e^-tau)) d / L, id = 1 / d [cm^-1] (calc_GH_tot.c:178-228).
+__device__ __forceinline__ void art_terms(const ArtCell &cl, float m1, float m2, float m3, const ArtStep &st,
+                                          float nswept, float id, float (&gh)[6]) {
+  const float j1 = fmaf(nswept, cl.s1, m1 / cl.a1 * id), j2 = fmaf(nswept, cl.s2, m2 / cl.a2 * id),
+              j3 = fmaf(nswept, cl.s3, m3 / cl.a3 * id);
+  gh[0] = fmaf(j3, (float)kRintJHI3, fmaf(j2, (float)kRintJHI2, j1)) * st.f[0];
+  gh[3] = fmaf(j3, (float)kRintHHI3, fmaf(j2, (float)kRintHHI2, j1)) * st.f[1];
+  gh[1] = fmaf(j3, (float)kRintJHeI3, j2) * st.f[2];
+  gh[4] = fmaf(j3, (float)kRintHHeI3, j2) * st.f[3];
+  gh[2] = j3 * st.f[4];
+  gh[5] = j3 * st.f[5];
+}
+
+// Beside the general march: a group's terms added to its totals and the
+// accumulator cleared for the next group.
+__global__ void __launch_bounds__(256) k_art_group(uint64_t n, float4 *__restrict__ acc,
+                                                  const ArtCell *__restrict__ cells, ArtStep st, float nswept,
+                                                  float id, float *__restrict__ gh6) {
+  for (uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < n; c += (uint64_t)gridDim.x * blockDim.x) {
+    const float4 v = acc[c];
+    acc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    float gh[6];
+    art_terms(load_cell(cells + c), v.x, v.y, v.z, st, nswept, id, gh);
+#pragma unroll
+    for (int s = 0; s < 6; s++) gh6[s * n + c] += gh[s];
+  }
+}
+
+// The six rates of a cell (calc_GH_tot.c:232-247).  tot6: the general march's
+// and the earlier groups' totals (kGeneral; nswept the angles of the last
+// group) or the earlier groups' sums (nswept all of them).
 template <bool kGeneral>
 __global__ void __launch_bounds__(256) k_art_close(uint64_t n, int ny, int nz, const float4 *__restrict__ acc,
                                                   const float4 *__restrict__ acc_t, const float *__restrict__ tot6,
@@ -649,7 +677,6 @@ __global__ void __launch_bounds__(256) k_art_close(uint64_t n, int ny, int nz, c
                                                   ArtStep st, float nswept, float id, float r_nang,
                                                   float *__restrict__ rates6) {
   for (uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < n; c += (uint64_t)gridDim.x * blockDim.x) {
-    const ArtCell cl = load_cell(cells + c);
     const float4 v = acc[c];
     float m1 = v.x, m2 = v.y, m3 = v.z;
     if (acc_t) {
@@ -663,15 +690,8 @@ __global__ void __launch_bounds__(256) k_art_close(uint64_t n, int ny, int nz, c
       m2 = tot6[n + c] + (m2 - tot6[4 * n + c]);
       m3 = tot6[2 * n + c] + (m3 - tot6[5 * n + c]);
     }
-    const float j1 = fmaf(nswept, cl.s1, m1 / cl.a1 * id), j2 = fmaf(nswept, cl.s2, m2 / cl.a2 * id),
-                j3 = fmaf(nswept, cl.s3, m3 / cl.a3 * id);
     float gh[6];
-    gh[0] = fmaf(j3, (float)kRintJHI3, fmaf(j2, (float)kRintJHI2, j1)) * st.f[0];
-    gh[3] = fmaf(j3, (float)kRintHHI3, fmaf(j2, (float)kRintHHI2, j1)) * st.f[1];
-    gh[1] = fmaf(j3, (float)kRintJHeI3, j2) * st.f[2];
-    gh[4] = fmaf(j3, (float)kRintHHeI3, j2) * st.f[3];
-    gh[2] = j3 * st.f[4];
-    gh[5] = j3 * st.f[5];
+    art_terms(load_cell(cells + c), m1, m2, m3, st, nswept, id, gh);
 #pragma unroll
     for (int s = 0; s < 6; s++) {
       if (kGeneral) gh[s] += tot6[s * n + c];
@@ -922,7 +942,8 @@ int art_run(const argot_b200_art *a, const ArtGeom &g, double denstonh, double u
   if (acc_t) ARGOT_CUDA_TRY(cudaMemsetAsync(acc_t, 0, sizeof(float4) * n, st));
   // groups of angles per launch: enough CTAs for kArtWaves fills of the GPU
   // and at least 128 angles; between groups the sums (of about 2 terms per
-  // angle) go into compensated totals
+  // angle) go into totals, compensated ones or the general march's
+  const float id = (float)(1.0 / ((double)std::min(g.dx, std::min(g.dy, g.dz)) * g.lunit));
   const uint64_t pairs = std::max<uint64_t>((uint64_t)((g.nx + 1) / 2) * std::max(g.ny, g.nz),
                                             (uint64_t)((g.ny + 1) / 2) * g.nz);
   const uint32_t tiles = (uint32_t)((pairs + kArtThreads - 1) / kArtThreads);
@@ -932,12 +953,15 @@ int art_run(const argot_b200_art *a, const ArtGeom &g, double denstonh, double u
     if (steps(i) == 0) continue;
     const int j = run_end(i);
     for (int a0 = i; a0 < j;) {
-      if (in_group >= group && !general) {
-        k_art_gather<<<blocks, 256, 0, st>>>(n, g.ny, g.nz, acc, acc_t, gh6);
+      if (in_group >= group) {
+        if (general)
+          k_art_group<<<blocks, 256, 0, st>>>(n, acc, cells, a->step, (float)in_group, id, gh6);
+        else
+          k_art_gather<<<blocks, 256, 0, st>>>(n, g.ny, g.nz, acc, acc_t, gh6);
         ARGOT_CUDA_TRY(cudaGetLastError());
         in_group = 0;
       }
-      const int na = std::min(std::min(j - a0, 32768), general ? 32768 : group - in_group);
+      const int na = std::min(std::min(j - a0, 32768), group - in_group);
       k_art_sweep<<<dim3(tiles, (unsigned)na), kArtThreads, sizeof(float4) * (size_t)most, st>>>(g, a->dev_ang, a0,
                                                                                                   cells, acc, cells_t,
                                                                                                   acc_t);
@@ -948,10 +972,9 @@ int art_run(const argot_b200_art *a, const ArtGeom &g, double denstonh, double u
     }
   }
   const float r_nang = (float)(1.0e0 / a->nang);
-  const float id = (float)(1.0 / ((double)std::min(g.dx, std::min(g.dy, g.dz)) * g.lunit));
   if (general)
-    k_art_close<true><<<blocks, 256, 0, st>>>(n, g.ny, g.nz, acc, acc_t, gh6, cells, a->step, (float)nswept, id, r_nang,
-                                             rates6);
+    k_art_close<true><<<blocks, 256, 0, st>>>(n, g.ny, g.nz, acc, acc_t, gh6, cells, a->step, (float)in_group, id,
+                                             r_nang, rates6);
   else
     k_art_close<false><<<blocks, 256, 0, st>>>(n, g.ny, g.nz, acc, acc_t, gh6, cells, a->step, (float)nswept, id, r_nang,
                                              rates6);

@@ -298,6 +298,44 @@ def test_art_rates_against_f64_march(cuda_ok, n, cell, tol):
     art.close()
 
 
+@pytest.mark.gpu
+def test_art_many_swept_directions_beside_general_ones(cuda_ok):
+    """12288 swept directions and one that takes the general march (its path
+    is longer than a CTA holds): the mean of the two passes by themselves.
+    The sums of 128 directions are closed one after another, so that what
+    rounds is some 100 FP32 additions and as many groups, 6e-8 sqrt(100) at
+    most; all 12288 in one FP32 sum would be off by 6e-8 sqrt(2 12288 / 3),
+    5e-6."""
+    import torch
+    from argot_b200 import _lib as L, diffuse as D
+    from argot_b200.workload import units
+    n = (2, 2, 700)
+    lunit, denstonh = units()
+    cell = float(np.float32(1.0 / 700))
+    box = [float(np.float32(k) * np.float32(cell)) for k in n]
+    g = L.Grid(*n, 0, 0, 0, 0.0, 0.0, 0.0, *box, 0.0, 0.0, 0.0, cell, cell, cell, lunit, denstonh)
+    nc = int(np.prod(n))
+    rng = np.random.default_rng(5)
+    f = torch.from_numpy(np.stack([_fields(1, int(rng.integers(1 << 30)))[:, 0] for _ in range(nc)], 1)).cuda()
+    dirs, bc, _ = D.angle_table(32)
+    long_dir, long_bc = _unit([[3, 2.9, 1]]), np.zeros((1, 2), np.int32)
+
+    def run(d, b):
+        art = D.Diffuse(table=(d, b, None))
+        r = torch.zeros(6 * nc, dtype=torch.float32, device="cuda")
+        art.rates(g, UENETOK, f, r)
+        L.check(L.load().argot_b200_check_device_error(torch.cuda.current_stream().cuda_stream), "device error")
+        art.close()
+        return r.double()
+
+    swept, general = run(dirs, bc), run(long_dir, long_bc)
+    both = run(np.concatenate([dirs, long_dir]), np.concatenate([bc, long_bc]))
+    want = (len(dirs) * swept + general) / (len(dirs) + 1)
+    assert torch.isfinite(want).all() and (want > 0).all()
+    err = (both - want) / want
+    assert err.square().mean().sqrt() < 6e-7
+
+
 def _coefficients(f, denstonh):
     """Absorption [cm^-1] and source functions of the three frequencies
     (calc_rmesh_data.c:33-111, diffuse_chemistry.c:13-103) in float64."""
