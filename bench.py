@@ -400,9 +400,10 @@ def compare_rate_modes(pb, rays, tau, prec, sur):
 # ------------------------------------------------------------ parity check
 def sampled_parity(pb, wl, sur, runs: int = 16, length: int = 16, seed: int = 11):
     """The checker on this workload: seeded runs of target cells computed by
-    the reference's own group loop (ARGOT's C, O1) and by the FP64 CPU
-    oracle pipeline (FP64 march + FP64 rates) on O1's rays, against the
-    device path on the target blocks holding them (oracle/sampled.py).
+    the reference's own group loop (ARGOT's C, O1, or its restatement where
+    that is not at hand) and by the FP64 CPU oracle pipeline (FP64 march + FP64
+    rates) on the same rays, against the device path on the target blocks
+    holding them (oracle/sampled.py).
     Reported per rate mode: the largest relative error per output field
     over the sampled cells; for the reference-order path its ray lists and
     columns against O1 and its FP64 rates against O1's."""
@@ -416,8 +417,7 @@ def sampled_parity(pb, wl, sur, runs: int = 16, length: int = 16, seed: int = 11
     r32, rays_k = sp.device(pb, L.PRECISION_KAHAN, L.RATE_EXACT_F32, want_rays=True)
     out = {"sample": (f"{runs} seeded runs of {length} consecutive target cells along z "
                       f"({len(sp.all_cells())} cells, {len(ref['tgt'])} rays)"),
-           "oracle": "O1 = ARGOT's C (reference order, FP32 march, FP64 rates); "
-                     "FP64 = orc_march_f64 + orc_photoion_f64 on O1's rays",
+           "oracle": sp.source + "; FP64 = orc_march_f64 + orc_photoion_f64 on the same rays",
            "reference_order": {"ray_lists_equal_O1": bool(same_list), "columns_bitwise_O1": bool(same_tau),
                                "exact_f64_rates_vs_O1": sp.rate_errors(r64, ref["rates"])},
            "kahan_columns_vs_fp64": sp.column_error_vs_f64(rays_k),
@@ -1073,10 +1073,12 @@ def main(argv=None):
         print(json.dumps({"config": wl.name,
                           "reference_gpu": reference_gpu_sample(wl, target_rays=args.reference_gpu_rays)}),
               flush=True)
-    elif args.impl == "reference" and args.config.startswith("art"):
-        run_reference_art(args)
     elif args.impl == "reference":
-        run_reference(args)
+        try:
+            (run_reference_art if args.config.startswith("art") else run_reference)(args)
+        except FileNotFoundError:
+            print(json.dumps({"impl": "reference", "unavailable": "ARGOT's sources are not at hand and no library "
+                              "prebuilt from them for this mesh"}), flush=True)
     elif args.config.startswith("art"):
         run_art(args)
     elif args.config.startswith("batched"):

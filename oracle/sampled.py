@@ -21,6 +21,11 @@ on the target blocks that contain them, and compares on the sampled cells:
 * the compensated (Kahan) columns against the FP64 march,
 * the FP32 and surrogate rates against the FP64 oracle pipeline.
 
+Where ARGOT's C is not at hand (no sources and no prebuilt library), the C
+restatement stands for it: the light rays of a restated tree walk
+(oracle/tree.py), the reference-order columns of ``orc_march_f32ref`` and the
+rates of ``orc_photoion_f64ref``.  ``source`` says which one compared.
+
 Only tests/, ``__graft_entry__.smoke`` and bench.py's checks import this
 module; the product never does.
 """
@@ -28,6 +33,7 @@ from __future__ import annotations
 
 import numpy as np
 
+from . import build as _build
 from .oracle import Oracle, RefLib, unit_box_grid
 
 NAMES = ("gamma_HI", "gamma_HeI", "gamma_HeII", "heat_HI", "heat_HeI", "heat_HeII")
@@ -72,6 +78,9 @@ class SampledParity:
         self.oracle = Oracle()
         self._ref = None
         self._f64 = None
+        self.has_reference = os.path.exists(_build.ref_lib_path(wl.edge)) or _build.reference_available()
+        self.source = ("O1 = ARGOT's C (reference order, FP32 march, FP64 rates)" if self.has_reference else
+                       "O1 not at hand: its restatement (NumPy tree walk, orc_march_f32ref, orc_photoion_f64ref)")
 
     # ------------------------------------------------------------ cells
     def _runs(self):
@@ -102,6 +111,9 @@ class SampledParity:
         columns, per-ray spectrum) and the cells' FP64 rates."""
         if self._ref is not None:
             return self._ref
+        if not self.has_reference:
+            self._ref = self._restated()
+            return self._ref
         wl = self.wl
         R = RefLib(wl.edge)
         R.init(wl.lunit, wl.denstonh, wl.theta, self.threads)
@@ -120,6 +132,36 @@ class SampledParity:
         self._ref["rates"] = np.concatenate(rates, axis=1)
         return self._ref
 
+    def _restated(self):
+        """the same from the restatement; the spectra once per emitter, with
+        each ray's index"""
+        from .tree import Tree
+        wl = self.wl
+        if wl.src_spectra is not None:
+            spec = np.asarray(wl.src_spectra, np.float64)
+        else:
+            spec = np.stack([self.oracle.photon_rate(t, p, r)
+                             for t, p, r in zip(wl.src_type, wl.src_param, wl.src_rate)])
+        tree = Tree(wl.src_pos, spec)
+        pos, spectra = tree.emitters()
+        side = np.float64(np.float32(1.0) / np.float32(self.edge))
+        parts = {k: [] for k in ("tgt", "src", "seg", "tau", "spec_index", "rates")}
+        for run in self._runs():
+            c = self.cells(run)
+            ijk = np.stack([c // self.edge ** 2, c // self.edge % self.edge, c % self.edge], 1)
+            centres = ((ijk + 0.5) * side).astype(np.float32)
+            cell, emit = tree.rays(centres, wl.theta)
+            r = {"tgt": ijk[cell].astype(np.int32), "src": pos[emit], "spec_index": emit.astype(np.uint64),
+                 "seg": np.concatenate([pos[emit], centres[cell]], 1)}
+            r["tau"] = self.oracle.march_f32ref(self.grid, wl.fields(), r["seg"])
+            r["rates"] = self.oracle.photoion_f64ref(self.grid, wl.fields(), r["tau"], r["tgt"], r["src"], spectra,
+                                                     r["spec_index"])[:, c]
+            for k, v in r.items():
+                parts[k].append(v)
+        out = {k: np.concatenate(v, axis=1 if k == "rates" else 0) for k, v in parts.items()}
+        out["spectra"] = spectra
+        return out
+
     # ------------------------------------------------------------ FP64 oracle
     def fp64(self):
         """The FP64 precision oracle on O1's rays of the sampled cells:
@@ -130,7 +172,7 @@ class SampledParity:
         ref = self.reference()
         t64 = self.oracle.march_f64(self.grid, self.wl.fields(), ref["seg"])
         r64 = self.oracle.photoion_f64(self.grid, self.wl.fields(), t64, ref["tgt"], ref["seg"][:, :3],
-                                       ref["spectra"])
+                                       ref["spectra"], ref.get("spec_index"))
         self._f64 = {"tau": t64, "rates": r64[:, self.all_cells()]}
         return self._f64
 
