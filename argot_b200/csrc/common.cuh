@@ -50,18 +50,13 @@ struct GridDev {
 GridDev make_grid(const argot_b200_grid &g);
 bool grid_valid(const argot_b200_grid *g);
 
-// Tables in constant memory (filled once per device by ensure_tables()).
+// Tables in constant memory.
 struct RateTables {
-  float nu_f[kNu];        // (float) nu, as the reference compares it
-  float cs[3][kNu];       // sigma_s(nu) [cm^2]
-  float cs_l2e[3][kNu];   // sigma_s(nu) * log2(e)
-  float hw[3][kNu];       // sigma_s(nu) * max((float)nu - nu_s, 0)
-  float hw_l2e[3][kNu];   // sigma_s(nu) * log2(e) * max((float)nu - nu_s, 0)
+  float cs[3][kNu];  // sigma_s(nu) [cm^2]
   // max of sigma_s(nu) over the bins k >= 64 m (the stages of the FP32 loop)
   float smax[3][4];
 };
-// Uploads the tables to the constant bank of the translation unit that owns
-// the rate kernels (photoion.cu), once per device.
+// Uploads the tables of the rate kernels (photoion.cu), once per device.
 int ensure_tables(int device);
 
 // Photo-ionisation cross sections [cm^2] at nu in units of the HI Lyman
