@@ -197,48 +197,6 @@ def test_art_dropin_through_mesh_dev(cuda_ok):
         assert np.array_equal(got["prev_chem"][f], before["prev_chem"][f])
 
 
-# ------------------------------------------------ the march in 64 bits
-def _march_f64(n, d, lunit, ab, S, dirs, faces):
-    """J_s = sum over directions of (sum over rays of I (1 - e^-tau)) /
-    (a_s sum of chords) + S_s per cell, float64: parallel rays from the cells
-    of each direction's start face, wrapped through the side faces with I
-    reset (ray_tracing.c, one isolated rank)."""
-    off = (0.521212345, 0.508512345, 0.468287655)
-    J = np.zeros(tuple(n) + (3,))
-    for o, base in zip(dirs.astype(np.float64), faces):
-        ax = (2, 2, 0, 0, 1, 1)[base]
-        p, q = [k for k in range(3) if k != ax]
-        num, chord = np.zeros(tuple(n) + (3,)), np.zeros(tuple(n))
-        for a in range(n[p]):
-            for b in range(n[q]):
-                i = [0, 0, 0]
-                i[p], i[q], i[ax] = a, b, (0 if base % 2 == 0 else n[ax] - 1)
-                x = [(i[k] + off[k]) * d[k] for k in range(3)]
-                x[ax] = 0.0 if base % 2 == 0 else n[ax] * d[ax]
-                nxt = [((i[k] + (o[k] > 0)) * d[k] - x[k]) / o[k] for k in range(3)]
-                I, s = np.zeros(3), 0.0
-                while True:
-                    m = min(nxt)
-                    c, idx = (m - s) * lunit, tuple(i)
-                    e = -np.expm1(-ab[idx] * c)
-                    num[idx] += I * e
-                    chord[idx] += c
-                    I = I * (1 - e) + S[idx] * e
-                    s = m
-                    for k in range(3):
-                        if nxt[k] == m:
-                            nxt[k] += d[k] / abs(o[k])
-                            i[k] += 1 if o[k] > 0 else -1
-                    if not 0 <= i[ax] < n[ax]:
-                        break
-                    for k in (p, q):
-                        if not 0 <= i[k] < n[k]:
-                            i[k] %= n[k]
-                            I = np.zeros(3)
-        J += num / (ab * np.where(chord > 0, chord, np.inf)[..., None]) + S
-    return J
-
-
 def _unit(v):
     v = np.asarray(v, np.float64)
     return (v / np.linalg.norm(v, axis=-1, keepdims=True)).astype(np.float32)
@@ -262,6 +220,7 @@ def test_art_rates_against_f64_march(cuda_ok, n, cell, tol):
     of one, and they add up along the path: 2e-3."""
     import torch
     from argot_b200 import _lib as L, diffuse as D
+    from oracle import art as ART
     vec, faces = _SWEPT
     if n[2] == 600:
         vec, faces = vec + [[3, 2.9, 1]], faces + [0]
@@ -284,17 +243,57 @@ def test_art_rates_against_f64_march(cuda_ok, n, cell, tol):
         got.zero_()
         art.rates(g, UENETOK, f, got, crossings=crossings)
     L.check(L.load().argot_b200_check_device_error(torch.cuda.current_stream().cuda_stream), "device error")
-    ab, S = _coefficients(planes.astype(np.float64), denstonh)
-    J = _march_f64(n, [float(np.float32(c)) for c in cell], lunit, ab.reshape(tuple(n) + (3,)),
-                   S.reshape(tuple(n) + (3,)), dirs, faces).reshape(nc, 3) / len(faces)
-    st = D.step_factors().astype(np.float64)
-    want = np.stack([(J @ [1, 1.128855608262e-01, 5.288790581895e-03]) * st[0], (J @ [0, 1, 1.2404369898e-01]) * st[2],
-                     J[:, 2] * st[4], (J @ [1, 3.1154224364e+00, 5.2452188546e-01]) * st[1],
-                     (J @ [0, 1, 8.7872474963e+00]) * st[3], J[:, 2] * st[5]])
+    want = ART.rates(n, [float(np.float32(c)) for c in cell], lunit, denstonh, UENETOK, planes, dirs, faces,
+                     D.step_factors())
     err = np.abs(got.view(6, -1).double().cpu().numpy() - want) / np.abs(want)
     assert err.max() < tol, err.max(axis=1)
     # every ray of a swept direction crosses at least one cell per layer
     assert int(cnt.item()) >= sum(nc for _ in _SWEPT[1])
+    art.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what", ["steep", "box", "leaving"])
+def test_art_odd_tables_and_boxes(cuda_ok, what):
+    """steep: directions whose start face is not the one of their largest
+    component (swept all the same).  box: a box that is not the local domain,
+    its upper side a hundredth of a cell off, where no direction is swept (no
+    ray here starts on that side, so the float64 march holds).  leaving: a
+    direction that does not enter through its start face crosses no cell, and
+    the mean over its crossings is undefined in all of them, as in the
+    reference's sums.  Against the float64 march on the local domain; the
+    general march's float positions leave 1e-5 on these meshes."""
+    import torch
+    from argot_b200 import _lib as L, diffuse as D
+    from argot_b200.workload import units
+    from oracle import art as ART
+    n, cell = (6, 5, 7), 0.125
+    lunit, denstonh = units()
+    vec, faces = [[1, 1.7, 3], [0.4, 0.2, 2], [2, 1, 0.9], [0.2, 3, 1.1]], [0, 0, 2, 4]
+    if what == "steep":
+        vec, faces = vec + [[2, 1.5, 0.4], [0.3, 0.5, 2]], faces + [0, 2]
+    elif what == "leaving":
+        vec, faces = vec + [[1, 1.5, -2]], faces + [0]
+    dirs = _unit(vec)
+    top = [k * cell + (0.01 * cell if what == "box" else 0.0) for k in n]
+    g = L.Grid(*n, 0, 0, 0, 0.0, 0.0, 0.0, *top, 0.0, 0.0, 0.0, cell, cell, cell, lunit, denstonh)
+    nc = int(np.prod(n))
+    rng = np.random.default_rng(11)
+    planes = np.stack([_fields(1, int(rng.integers(1 << 30)))[:, 0] for _ in range(nc)], 1)
+    bc = np.zeros((len(faces), 2), np.int32)
+    bc[:, 0] = faces
+    f = torch.from_numpy(planes).cuda()
+    art = D.Diffuse(table=(dirs, bc, None))
+    for apass in (1, 3, 8):
+        got = torch.zeros(6 * nc, dtype=torch.float32, device="cuda")
+        art.rates(g, UENETOK, f, got, angles_per_pass=apass)
+        L.check(L.load().argot_b200_check_device_error(torch.cuda.current_stream().cuda_stream), "device error")
+        if what == "leaving":
+            assert torch.isnan(got).all()
+            continue
+        want = ART.rates(n, [cell] * 3, lunit, denstonh, UENETOK, planes, dirs, faces, D.step_factors())
+        err = np.abs(got.view(6, -1).double().cpu().numpy() - want) / np.abs(want)
+        assert err.max() < 1e-5, (apass, err.max(axis=1))
     art.close()
 
 
@@ -334,42 +333,3 @@ def test_art_many_swept_directions_beside_general_ones(cuda_ok):
     assert torch.isfinite(want).all() and (want > 0).all()
     err = (both - want) / want
     assert err.square().mean().sqrt() < 6e-7
-
-
-def _coefficients(f, denstonh):
-    """Absorption [cm^-1] and source functions of the three frequencies
-    (calc_rmesh_data.c:33-111, diffuse_chemistry.c:13-103) in float64."""
-    dens, hi, hii, hei, heii, heiii, fe, u = f
-    he = 0.0811258278
-    t = np.maximum(u * UENETOK / ((1 + fe) * 0.755 + 0.25 * 0.245), 1.0)
-    nh = dens * denstonh
-    ne = nh * (hii + he * (heii + 2 * heiii))
-
-    def sig(s, v):
-        thr = (1.0, 1.8125, 4.0)[s]
-        if s == 1:
-            return 7.83e-18 * (1.66 * (v / thr) ** -2.05 - 0.66 * (v / thr) ** -3.05)
-        e = np.sqrt(v / thr - 1.0)
-        return 6.3e-18 * (1.0, 0, 64.0)[s] / v ** 4 * np.exp(4 - 4 * np.arctan(e) / e) / (1 - np.exp(-2 * np.pi / e))
-
-    cs = [float(np.float32(sig(s, (1.0, 1.8125, 4.0)[s] + 1e-7))) for s in range(3)]
-    k = [cs[0] * hi * nh, cs[1] * he * hei * nh, cs[2] * he * heii * nh]
-    ab = np.stack([k[0], k[0] * 1.9529766579e-01 + k[1], k[0] * 1.9513732355e-02 + k[1] * 2.6858709594e-01 + k[2]], -1)
-    ab = ab + 1e-31
-    l, tev = np.log(t * 8.61623e-5), t * 8.61623e-5
-    p = np.polyval([-3.071135243196595e-9, -1.856767039775261e-8, 5.755614137575758e-7, 4.989108920299513e-6,
-                    -0.00001421502914054107, -0.0003212605213188796, -0.002380861877349834, -0.02026044731984691,
-                    -0.7241125657826851, -28.61303380689232], l)
-
-    def b(lam, a):
-        return a * lam ** 1.5 / (1 + (lam / 2.740) ** 0.407) ** 2.242
-
-    low = 3.92e-13 / tev ** 0.6353
-    hot = 1.54e-9 * (1 + 0.3 / np.exp(8.099328789667 / tev)) / (np.exp(40.49664394833662 / tev) * tev ** 1.5)
-    he2a = np.where(tev > 0.8, hot + low, low)
-    he2b = np.where(t > 500.3, 1.26e-14 * (2 * 285335.0 / t) ** 0.75, (1.12e-10 - 2.1e-11 * np.log10(t)) / np.sqrt(t))
-    he3a = 3.36e-10 / np.sqrt(t) / (t / 1e3) ** 0.2 / (1 + (t / 1e6) ** 0.7)
-    rec = (np.exp(p) - b(2 * 157807.0 / t, 2.753e-14), he2a - he2b, he3a - b(2 * 631515.0 / t, 1.3765e-14))
-    ion = (hii * nh, he * heii * nh, he * heiii * nh)
-    e = np.stack([r * ne * x * 13.6 * w * 1.6022e-12 / (4 * np.pi) for r, x, w in zip(rec, ion, (1.0, 1.8125, 4.0))], -1)
-    return ab, e / ab
