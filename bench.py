@@ -13,7 +13,7 @@ target throughput is quoted.  Inputs (13 GB of rays + a 268 MB field) are
 larger than the 126 MB L2, so no flush is needed between steps.
 
 metric: ray-cell crossings/s of the whole step; the JSON line also carries
-Gamma-cells/s, the per-kernel split, a roofline object for the march (HBM
+Gamma-cells/s, the per-kernel split, a roofline object for the march (L1
 bound) and the reference's CPU path timed on a bounded sample.
 
 Usage: python bench.py [--gpus N] [--steps K] [--warmup W]
@@ -40,14 +40,16 @@ CONFIGS = ("largest", "plain", "precision", "learned", "tiny", "plain256", "batc
 ART_METRIC = "ART diffuse ray-cell steps/s (768 HEALPix directions, 1 B200)"
 ART_UENETOK = 1.0e4
 METRIC = "ray-cell crossings/s (march+stitch+rates, 1 B200)"
-# DRAM bytes per ray-cell crossing of k_march_rays<Kahan> measured by ncu on
-# the 256^3 / 16-source case (dram__bytes_read.sum + dram__bytes_write.sum =
-# 104.7 + 17.4 GB over a 104.1 ms launch for 6.030e10 crossings); the
-# workloads here are too large to capture, so `traffic` scales this figure.
-MARCH_DRAM_BYTES_PER_CROSSING = 2.024
-# the same capture's L2 bytes (lts__t_sectors.sum x 32 B, 413.0 GB over the
-# launch's 6.030e10 crossings): what the L2 serves per crossing
-MARCH_L2_BYTES_PER_CROSSING = 6.848
+# DRAM and L2 bytes per ray-cell crossing of k_march_rays<Kahan> measured by
+# ncu on 224^3 cells / 32 clustered sources (dram__bytes_read.sum +
+# dram__bytes_write.sum = 27.8 + 11.5 GB, lts__t_sectors.sum x 32 B = 287 GB,
+# over 5.184e10 crossings in 78.2 ms); the workloads here are too large to
+# capture, so `traffic` scales these figures.
+MARCH_DRAM_BYTES_PER_CROSSING = 0.758
+MARCH_L2_BYTES_PER_CROSSING = 5.53
+# DRAM bytes per ray-cell step of k_art_sweep by ncu at 128^3 (2.29 + 0.87 GB in
+# the launch of 128 of the 768 directions, 4.98e8 steps)
+ART_DRAM_BYTES_PER_STEP = 6.35
 UNIT = "crossings/s"
 
 
@@ -95,6 +97,19 @@ def measured_peaks():
             d = json.load(f)
         return float(d["hbm_gbs"]), float(d["bf16_tflops"]), "measured"
     return 6650.0, 1590.0, "fallback"
+
+
+def l1_roofline(kernel: str, nbytes: float, seconds: float, sm_mhz: float | None) -> dict:
+    """bytes that a kernel's lanes take from L1 against what the L1s deliver:
+    128 bytes per clock and SM at the device's highest clock (None, no clock
+    sample: the B200's 1965 MHz)"""
+    import torch
+    sm_mhz = sm_mhz or 1965.0
+    sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+    peak = sms * 128 * sm_mhz * 1e-3
+    achieved = nbytes / seconds / 1e9
+    return {"kernel": kernel, "bound": "l1", "achieved": achieved, "peak": peak, "unit": "GB/s",
+            "frac": achieved / peak, "peak_kind": f"nominal: {sms} SMs x 128 B x {sm_mhz:.0f} MHz"}
 
 
 def workload_config(wl, ws: int, sharded: bool) -> dict:
@@ -553,7 +568,6 @@ def run_ours(args):
 
     hbm, bf16, peak_kind = measured_peaks()
     alg_bytes = 16.0 * n_cross + 36.0 * nray_mine
-    achieved = alg_bytes / t_march / 1e9
     launches_per_step = (2 * pb.part_count(overlap) if overlap > 1
                          else len(pb.groups) * (2 + (0 if single else 1)))
 
@@ -584,21 +598,20 @@ def run_ours(args):
                   "rates_gamma_cells_per_s": ncell_mine / t_rates,
                   "rates_rays_per_s": nray_mine / t_rates,
                   "smooth_s": t_smooth, "smooth_gb_per_s": 2 * 24 * pb.ncell / t_smooth / 1e9},
-        "roofline": {"kernel": "k_march_rays", "bound": "hbm", "achieved": achieved,
-                     "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
-                     "peak_kind": f"{peak_kind} hbm_gbs",
+        "roofline": {**l1_roofline("k_march_rays", 16.0 * n_cross, t_march, clk["sm_max_mhz"]),
                      "traffic": MARCH_DRAM_BYTES_PER_CROSSING * n_cross,
                      "l2_traffic": MARCH_L2_BYTES_PER_CROSSING * n_cross,
-                     "traffic_source": (f"ncu DRAM bytes per crossing on 256^3 / 16 sources "
+                     "traffic_source": (f"ncu DRAM bytes per crossing on 224^3 / 32 sources "
                                         f"({MARCH_DRAM_BYTES_PER_CROSSING} B; L2 {MARCH_L2_BYTES_PER_CROSSING} B), "
                                         f"scaled by this launch's crossings"),
                      "dram_gbs": MARCH_DRAM_BYTES_PER_CROSSING * n_cross / t_march / 1e9,
                      "dram_frac": MARCH_DRAM_BYTES_PER_CROSSING * n_cross / t_march / 1e9 / hbm,
-                     "limiter": ("latency of the L1/L2-hit gathers (ncu: long-scoreboard stalls 14.1 per issue, "
-                                 "issue active 60%); DRAM moves 2.0 B and L2 serves 6.8 B of the 16 B per "
-                                 "crossing that the bytes model counts"),
+                     "dram_peak_kind": f"{peak_kind} hbm_gbs",
+                     "limiter": ("the L1 data pipe (ncu: 75% of its cycles; a warp's 16-byte gather touches 10 lines, "
+                                 "one per cycle), beside issue 70% and the ALU 66%"),
                      "algorithmic_bytes": alg_bytes,
-                     "bytes_model": "16 B per crossing + 36 B per ray"},
+                     "bytes_model": "achieved: 16 B per crossing from L1; algorithmic: 16 B per crossing + 36 B per "
+                                    "ray"},
         "clocks": clk,
         "gpu_launches": launches_per_step * args.steps,
     }
@@ -729,9 +742,7 @@ def run_batched(args):
     t = allmax(ws, e0.elapsed_time(e1) / 1e3, dev)
     total_cross = allsum(ws, float(n_cross) * args.steps, dev)
     total_cells = allsum(ws, float(B.ncell) * args.steps, dev)
-    hbm, _, peak_kind = measured_peaks()
     alg_bytes = 16.0 * n_cross + 24.0 * B.nray
-    achieved = alg_bytes / (t / args.steps) / 1e9 if ws == 1 else None
     e2e = None if args.no_e2e else batched_e2e(B, wls, dev, steps=max(1, min(args.steps, 3)))
     if e2e is not None:
         cross = e2e.pop("_crossings")
@@ -745,18 +756,21 @@ def run_batched(args):
                                f"{sorted(set(w.edge for w in wls))}, sources "
                                f"{min(w.nsrc for w in wls)}-{max(w.nsrc for w in wls)}",
                    "rays": B.nray, "crossings": n_cross, "cells": B.ncell,
-                   "launch": "one persistent kernel per step, replayed as a CUDA graph",
+                   "launch": ("one persistent kernel per step" if cfg["mode"] == 0 else
+                              f"two persistent kernels per part, {cfg['parts']} parts, per step")
+                   + ", replayed as a CUDA graph",
                    "autotuned": cfg, "tune_best_ms": tune_ms,
                    "l2": f"inputs larger than L2 ({B.nray * 4 / 1e9:.1f} GB rays); no flush",
                    "parallelism": f"{ws} independent batches (one per GPU)"},
         "gamma_cells_per_s": total_cells / t,
-        "roofline": {"kernel": "k_batch (march + rates fused)", "bound": "hbm", "achieved": achieved,
-                     "peak": hbm, "unit": "GB/s", "frac": achieved / hbm if achieved else None,
-                     "peak_kind": f"{peak_kind} hbm_gbs", "traffic": None,
-                     "algorithmic_bytes": alg_bytes,
-                     "bytes_model": "16 B per crossing + 24 B per ray (end points; columns stay on chip)"},
+        "roofline": {**l1_roofline("k_batch (march + rates fused)" if cfg["mode"] == 0 else
+                                   "k_batch_march + k_batch_rates (overlapped parts)",
+                                   16.0 * n_cross, t / args.steps, clk["sm_max_mhz"]),
+                     "traffic": None, "algorithmic_bytes": alg_bytes,
+                     "bytes_model": "achieved: 16 B per crossing from L1; algorithmic: 16 B per crossing + 24 B per "
+                                    "ray (end points, and the columns through HBM)"},
         "clocks": clk,
-        "gpu_launches": args.steps,
+        "gpu_launches": (1 if cfg["mode"] == 0 else 2 * cfg["parts"]) * args.steps,
     }
     if e2e is not None:
         line["e2e"] = e2e
@@ -891,15 +905,12 @@ def run_art(args):
     t = allmax(ws, e0.elapsed_time(e1) / 1e3, dev)
     total = allsum(ws, float(steps_per_pass) * args.steps, dev)
     hbm, _, peak_kind = measured_peaks()
-    # algorithmic bytes of one pass: per step two float4 of cell data read
-    # and one float4 reduction (from and to L2); per cell 8 planes in, 6
-    # planes of totals and 6 rate planes
-    alg = 48.0 * steps_per_pass + 4.0 * n * (8 + 6 + 12)
     # launches: cells, the sweeps of the directions in groups with a gather
     # between two, the closing kernel (csrc/art.cu art_run)
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
     tiles = -(-((wl.edge + 1) // 2 * wl.edge) // 128)
-    groups = -(-art.nang // max(128, -(-4 * 148 * 7 // tiles)))
-    achieved = alg / (t / args.steps) / 1e9
+    groups = -(-art.nang // max(128, -(-4 * sms * 7 // tiles)))
+    sec = t / args.steps
     # e2e: the 8 planes from pinned host memory, the pass, the rates back
     pin_f = torch.from_numpy(planes).pin_memory()
     out = torch.empty(6 * n, dtype=torch.float32).pin_memory()
@@ -926,10 +937,15 @@ def run_art(args):
                    "angles_per_pass": apass, "steps_per_pass": steps_per_pass,
                    "l2": "cell data 1 GB at 256^3, 134 MB at 128^3 (both layouts); no flush",
                    "parallelism": f"{ws} independent meshes (one per GPU)"},
-        "roofline": {"kernel": "k_art_cells + k_art_sweep + k_art_gather + k_art_close (one pass)", "bound": "hbm",
-                     "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
-                     "peak_kind": f"{peak_kind} hbm_gbs", "traffic": None,
-                     "bytes_model": "48 B per ray-cell step (served by L1 and L2) + 104 B per cell"},
+        "roofline": {**l1_roofline("k_art_cells + k_art_sweep + k_art_gather + k_art_close (one pass)",
+                                   32.0 * steps_per_pass, sec, clk["sm_max_mhz"]),
+                     "traffic": ART_DRAM_BYTES_PER_STEP * steps_per_pass,
+                     "traffic_source": f"ncu DRAM bytes per step at 128^3 ({ART_DRAM_BYTES_PER_STEP} B)",
+                     "dram_frac": ART_DRAM_BYTES_PER_STEP * steps_per_pass / sec / 1e9 / hbm,
+                     "dram_peak_kind": f"{peak_kind} hbm_gbs",
+                     "limiter": ("the L1 data pipe (ncu: 77% of its cycles, cell loads, reductions and the sums passed "
+                                 "between lanes), beside issue 70% and the heavy FMA pipe 48%"),
+                     "bytes_model": "32 B of cell data per ray-cell step from L1"},
         "e2e": {"value": float(steps_per_pass) / te, "unit": UNIT, "h2d_bytes_per_step": int(planes.nbytes),
                 "d2h_bytes_per_step": int(6 * n * 4), "s_per_step": te},
         "clocks": clk,
