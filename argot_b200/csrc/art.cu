@@ -737,14 +737,8 @@ __global__ void __launch_bounds__(256) k_art_to_mesh(uint64_t n, const float *__
 
 #endif  // ARGOT_HELIUM_LAYOUT
 
-int art_sms() {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
 int art_blocks(uint64_t n) {
-  const int sms = art_sms();
+  const int sms = device_sms();
   const uint64_t want = (n + 255) / 256;
   return (int)(want < (uint64_t)sms * 8 ? (want ? want : 1) : (uint64_t)sms * 8);
 }
@@ -952,7 +946,7 @@ int art_run(const argot_b200_art *a, const ArtGeom &g, double denstonh, double u
   const uint64_t pairs = std::max<uint64_t>((uint64_t)((g.nx + 1) / 2) * std::max(g.ny, g.nz),
                                             (uint64_t)((g.ny + 1) / 2) * g.nz);
   const uint32_t tiles = (uint32_t)((pairs + kArtThreads - 1) / kArtThreads);
-  const int group = (int)std::max<uint64_t>(128, (kArtWaves * art_sms() * kArtCtas + tiles - 1) / tiles);
+  const int group = (int)std::max<uint64_t>(128, (kArtWaves * device_sms() * kArtCtas + tiles - 1) / tiles);
   int in_group = 0;
   for (int i = 0, left = nswept; left > 0; i = run_end(i)) {
     if (steps(i) == 0) continue;

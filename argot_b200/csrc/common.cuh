@@ -47,6 +47,10 @@ struct GridDev {
   int pce;
 };
 
+// SMs of the current device (a small call asks on every launch otherwise,
+// 0.2 us each time).
+int device_sms();
+
 GridDev make_grid(const argot_b200_grid &g);
 bool grid_valid(const argot_b200_grid *g);
 

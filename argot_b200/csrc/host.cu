@@ -2,6 +2,7 @@
 // identification, the frequency/cross-section tables, source spectra and the
 // oct-tree over the sources.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -131,6 +132,16 @@ static double midpoint_stages(int type, double p, double a, double b) {
     prev = s;
   }
   return s;
+}
+
+int device_sms() {
+  static std::atomic<int> known[64];
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) != cudaSuccess) return sms;
+  if (dev < 64 && (sms = known[dev].load(std::memory_order_relaxed)) > 0) return sms;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+  if (dev < 64) known[dev].store(sms, std::memory_order_relaxed);
+  return sms;
 }
 
 }  // namespace argot

@@ -29,9 +29,7 @@ __global__ void k_pack_fields(uint64_t n, const float *__restrict__ dens, const 
 
 static int grid_blocks_for(uint64_t n, int threads) {
   uint64_t b = (n + threads - 1) / threads;
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const uint64_t cap = (uint64_t)sms * 16;
+  const uint64_t cap = (uint64_t)device_sms() * 16;
   return (int)(b < cap ? (b ? b : 1) : cap);
 }
 
@@ -508,9 +506,7 @@ int argot_b200_march_rays(const argot_b200_grid *gp, const void *packed, const a
   cudaStream_t st = (cudaStream_t)stream;
   // segments per block: enough items for kMarchItems per warp slot, at most
   // one per chunk of 32 rays of an average block
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const uint64_t nblk = b1 - b0, slots = 64ull * sms;
+  const uint64_t nblk = b1 - b0, slots = 64ull * device_sms();
   uint64_t nseg = std::min((kMarchItems * slots + nblk - 1) / nblk, (nray / nblk + 31) / 32);
   nseg = std::max<uint64_t>(1, std::min<uint64_t>(nseg, 64));
   const bool wide = nblk * nseg >= slots;

@@ -305,9 +305,7 @@ int launch_rate_f32_served(const GridDev &g, const float4 *raw, const float4 *em
 
 int grid_blocks_for_rates(uint64_t n, int threads) {
   uint64_t b = (n + threads - 1) / threads;
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const uint64_t cap = (uint64_t)sms * 16;
+  const uint64_t cap = (uint64_t)device_sms() * 16;
   return (int)(b < cap ? (b ? b : 1) : cap);
 }
 
@@ -343,8 +341,7 @@ extern "C" int argot_b200_photoion_rays(const argot_b200_grid *gp, const void *p
   cudaStream_t st = (cudaStream_t)stream;
   const int threads = 32 * kRateWarps;
   const int blocks = grid_blocks_for_rates((b1 - b0) * 32, threads);
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = device_sms();
   if (mode == ARGOT_B200_RATE_EXACT_F64)
     k_rate_blocks<<<blocks, threads, 0, st>>>(g, raw, t->emit_pos, t->emit_spec64, b0, b1, blk_off, base, rays,
                                               nray, tau, rates6, err);

@@ -178,8 +178,7 @@ int launch_smooth_planes(int nx, int ny, int nz, const float *in, float *out, in
                          cudaStream_t st) {
   const uint64_t ncell = (uint64_t)nx * ny * nz;
   if (!ncell || nplanes <= 0) return 0;
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = device_sms();
   // shorter segments where the mesh would leave the GPU's warps idle
   const uint64_t columns = (uint64_t)((ny + 1) / 2) * ((nz + 31) / 32), slots = kSmoothWarps * sms;
   int run = kRun;
