@@ -441,9 +441,10 @@ __device__ __forceinline__ void att_y2(float2 y, float2 *et, float2 *em1) {
 // with its per-angle accumulators, 64 angles at a time, took 33.4 ms and moved
 // 52 GB of accumulators through DRAM.  On the way: one ray per thread 12.1
 // ms, one reduction per crossing 12.5 ms (the path of the reductions to L2
-// busy 81%), without the copy with y fastest 17.0 ms.  What bounds it now:
-// issue (70%), the heavy FMA pipe (55%) and the latency of the cell loads at
-// 28 warps per SM.  Launch shape: 128 threads, 7 CTAs per SM; 6: 11.1 ms, 256
+// busy 81%), without the copy with y fastest 17.0 ms (15.0 ms now).  What bounds
+// it now (ncu, 128 directions): the L1 data pipe (77%: cell loads, reductions,
+// the sums passed between lanes), issue (70%) and the latency of the cell loads
+// at 28 warps per SM; the heavy FMA pipe stands at 48%, DRAM at 28%.  Launch shape: 128 threads, 7 CTAs per SM; 6: 11.1 ms, 256
 // threads x 3: 12.8 ms.
 __global__ void __launch_bounds__(kArtThreads, kArtCtas)
     k_art_sweep(ArtGeom g, const ArtAngle *__restrict__ ang, int a0, const ArtCell *__restrict__ cells,

@@ -140,13 +140,14 @@ __global__ void __launch_bounds__(256) k_walk(GridDev g, const DevNode *__restri
 // lie together walk the same cells.  Blocks are therefore taken in tiles
 // (block_of_item): two CTAs of 16 warps hold 2 x 4 x 4 blocks (4 x 16 x 16
 // cells), consecutive CTAs 8 x 8 x 8 blocks, instead of a row of blocks along
-// z.  ncu, 224^3 cells / 32 sources: L1 sector hits 37% -> 56%, L2 63% -> 89%,
-// DRAM no longer read 64 GB per launch, 82.9 -> 72.5 ms; 256^3 / 1024
-// clustered sources: 0.697 s -> 0.610 s with CTAs of 32 warps, 0.629 s with 16,
-// 0.664 s with 8; but the step that runs it beside the rates takes 0.990,
-// 0.975 and 0.983 s, so 16.  What bounds it now: the L1 data pipe (77% of its peak,
-// one line per cycle for each quarter warp of a 16-byte gather), the ALU
-// (68%) and issue (71%) together.
+// z.  ncu, 224^3 cells / 32 sources (2.6e8 rays), row by row in CTAs of 8 warps,
+// in tiles with CTAs of 16 and of 32: L1 sector hits 37%, 39% and 56%, L2 63%, 79%
+// and 89%, 82.9, 78.2 and 72.5 ms.  256^3 / 1024 clustered sources: 0.697 s row
+// by row, 0.610 s in tiles with CTAs of 32 warps, 0.629 s with 16, 0.664 s with 8;
+// but the step that runs it beside the rates takes 0.990, 0.975 and 0.983 s, so
+// 16.  What bounds it now: the L1 data pipe (75% of its peak: a warp's 16-byte
+// gather touches 10 lines, one per cycle, where 4 is the least), issue (70%) and
+// the ALU (66%) together.
 // Launch shape: 64 warps per SM (32 registers) in CTAs of 16 warps.  A range
 // of few blocks is cut finer: each block's chunks of 32 rays into segments,
 // one warp each, until there are kMarchItems items per warp slot (32^3 cells

@@ -93,8 +93,8 @@ constexpr float kHNuLf = (float)kHNuL;
 // The FP32 parameters of a ray from emitter (sx, sy, sz) to the centre of
 // target cell (gix, giy, giz) (global indices) with code-unit columns t_s;
 // raw = {dens, fHI, fHeI, fHeII} of the target cell.  A ray that starts at
-// its target's centre (r = 0) contributes nothing, as in the reference,
-// whose shell volume then diverges.
+// its target's centre (r = 0) contributes nothing here (the reference's
+// operations, and the FP64 rates, leave infinite and undefined rates there).
 __device__ __forceinline__ RayParams ray_params_f32(const GridDev &g, int gix, int giy, int giz, float sx,
                                                     float sy, float sz, float t0, float t1, float t2, float4 raw,
                                                     double total) {
@@ -134,16 +134,18 @@ __device__ __forceinline__ RayParams ray_params_f32(const GridDev &g, int gix, i
 // Stage 0 ends below the HeII threshold (bin 102), so it has no HeII terms;
 // they would add exact zeros.
 //
-// What bounds it: the heavy FMA pipe.  A ray takes 62 and 64 packed
-// operations in the two thin forms, 69 in form 2 and 70 to 72 beyond, at 2.1 cycles
-// (f32x2 operations issue on that pipe only) and about a dozen scalar ones:
-// about 150 cycles of the 205 it takes per SM sub-partition, counted from the code.  Before, four 8-lane groups per warp integrated two rays
-// each and read every bin pair's 48-byte table entry from shared memory and
-// its spectrum from global memory: 145 instructions and 41 L1 data-pipe
-// cycles per ray (63% of that pipe, of which the march beside it needs 77%)
-// against 130 and 23 now.  256^3 cells, 1024 clustered sources, 2.17e9 rays:
-// 0.524 s before, 0.471 s now.  Two rays at a time per warp (for more
-// independent chains): 0.461 s alone, the step with the march no faster.
+// What bounds it: the heavy FMA pipe (62% of its cycles; issue 59%, 16 warps per
+// SM) and waits between dependent operations.  A ray takes 62 and 64 packed
+// operations in the two thin forms, 69 in form 2 and 70 to 72 beyond, at 2.1
+// cycles (f32x2 operations issue on that pipe only) and about a dozen scalar
+// ones: about 150 cycles per SM sub-partition, counted from the code, of 245
+// in the capture (224^3 cells / 32 sources, 2.6e8 rays, 54.9 ms).  Before, four
+// 8-lane groups per warp integrated two rays each and read every bin pair's
+// 48-byte table entry from shared memory and its spectrum from global memory: 145
+// instructions and 41 L1 data-pipe cycles per ray (that pipe is the march's
+// beside it) against 143 and 25 now.  256^3 cells, 1024 clustered sources, 2.17e9
+// rays: 0.527 s before, 0.480 s now.  Two rays at a time per warp (for more
+// independent chains): 2% faster alone, the step with the march no faster.
 // (RateShared reads them from a copy in shared memory instead, for a kernel
 // that needs its registers.)
 struct RateLane {

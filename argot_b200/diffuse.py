@@ -74,7 +74,9 @@ class Diffuse:
 
     def default_pass(self, grid, budget_bytes: int = 2 << 30) -> int:
         """angles per pass: about a million rays in flight, accumulators
-        within budget_bytes"""
+        within budget_bytes (sized for the general march; a table whose
+        directions are all swept uses four planes at most, and is slower with
+        fewer, see argot_b200_art_workspace)"""
         n = grid.nx * grid.ny * grid.nz
         face = max(grid.nx * grid.ny, grid.ny * grid.nz, grid.nz * grid.nx)
         a = max(1, min(self.nang, (1 << 20) // face))

@@ -501,7 +501,13 @@ ARGOT_B200_API int argot_b200_art_create(const float *dir3, const int *base_corn
 ARGOT_B200_API void argot_b200_art_destroy(argot_b200_art *a);
 ARGOT_B200_API int argot_b200_art_num_angles(const argot_b200_art *a);
 /* device workspace bytes for argot_b200_art_rates with angles_per_pass (the
- * workspace must be 32-byte aligned, as cudaMalloc returns it) */
+ * workspace must be 32-byte aligned, as cudaMalloc returns it).
+ * angles_per_pass: accumulator planes, one per direction that the general
+ * march takes at a time.  A table whose directions are all swept (each enters
+ * through its start face, the box is the local domain) needs one plane and
+ * uses up to four: from 4 on a copy of the cells with y fastest lies in them,
+ * which makes the pass a quarter to two fifths faster (128^3 cells 11.0 instead
+ * of 15.0 ms, 64^3 1.2 instead of 2.0). */
 ARGOT_B200_API uint64_t argot_b200_art_workspace(const argot_b200_grid *g, int angles_per_pass);
 /* fields8_dev: 8 planes of ncell floats: dens, fHI, fHII, fHeI, fHeII,
  * fHeIII, felec, uene (fluid_mesh dens, prev_chem fractions, prev_uene);
