@@ -81,9 +81,9 @@ class Batch:
         L.check(self.lib.argot_b200_check_device_error(self.sp), "device error flag")
 
     def close(self):
-        if self.handle:
-            self.lib.argot_b200_batch_free(self.handle)
-            self.handle = C.c_void_p()
+        handle, self.handle = self.handle, None
+        if handle:
+            self.lib.argot_b200_batch_free(handle)
         for pb in self.problems:
             pb.close()
 

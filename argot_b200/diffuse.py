@@ -62,9 +62,9 @@ class Diffuse:
         self._work = None
 
     def close(self):
-        if self.h:
-            self.lib.argot_b200_art_destroy(self.h)
-            self.h = None
+        h, self.h = self.h, None
+        if h:
+            self.lib.argot_b200_art_destroy(h)
 
     def __del__(self):
         try:

@@ -271,12 +271,13 @@ class Problem:
         return rates6
 
     def close(self):
-        if self._dtree:
-            self.lib.argot_b200_dev_tree_free(self._dtree)
-            self._dtree = C.c_void_p()
-        if self._tree:
-            self.lib.argot_b200_tree_free(self._tree)
-            self._tree = C.c_void_p()
+        # forgotten before they are freed: at interpreter exit this may run with
+        # the module's names gone, and once more from a batch's close
+        (dtree, self._dtree), (tree, self._tree) = (self._dtree, None), (self._tree, None)
+        if dtree:
+            self.lib.argot_b200_dev_tree_free(dtree)
+        if tree:
+            self.lib.argot_b200_tree_free(tree)
 
     def __del__(self):
         try:

@@ -72,9 +72,9 @@ class Surrogate:
         return cls(p, e, tol)
 
     def close(self):
-        if self.handle:
-            self.lib.argot_b200_surrogate_free(self.handle)
-            self.handle = C.c_void_p()
+        handle, self.handle = self.handle, None
+        if handle:
+            self.lib.argot_b200_surrogate_free(handle)
 
     def __del__(self):
         try:
