@@ -452,14 +452,16 @@ int launch_split(argot_b200_batch *b, unsigned long long *crossings, cudaStream_
     ARGOT_CUDA_TRY(cudaEventRecord(b->ev[1 + p], st));
     ARGOT_CUDA_TRY(cudaStreamWaitEvent(side, b->ev[1 + p], 0));
     const uint64_t nblk = b->item_blk[i1] - b->item_blk[i0];
-    if (cta_per_block(nblk, b->item_ray[i1] - b->item_ray[i0], (uint64_t)b->grid_rates_cta, kSplitRateWarps))
-      k_batch_rates_cta<<<(unsigned)std::min<uint64_t>(nblk, b->grid_rates_cta),  // (one unit per block)
-                          32 * kSplitRateWarps, 0, side>>>(b->probs_dev, b->items_dev, i0, i1,
-                                                           (uint32_t)b->cfg.blocks_per_item,
-                                                           b->counters + 2 * p + 1);
-    else
+    if (cta_per_block(nblk, b->item_ray[i1] - b->item_ray[i0], (uint64_t)b->grid_rates_cta, kSplitRateWarps)) {
+      uint64_t longest = 1;  // a unit per block of the longest tile, most of them empty in short ones: at most 256
+      for (uint32_t i = i0; i < i1; i++) longest = std::max(longest, b->item_blk[i + 1] - b->item_blk[i]);
+      k_batch_rates_cta<<<(unsigned)std::min<uint64_t>(nblk, b->grid_rates_cta), 32 * kSplitRateWarps, 0, side>>>(
+          b->probs_dev, b->items_dev, i0, i1, (uint32_t)std::min<uint64_t>(longest, 256),
+          b->counters + 2 * p + 1);
+    } else {
       k_batch_rates<<<b->grid_rates, 32 * kSplitRateWarps, 0, side>>>(
           b->probs_dev, b->items_dev, i0, i1, units(b->grid_rates * kSplitRateWarps), b->counters + 2 * p + 1);
+    }
     ARGOT_CUDA_TRY(cudaGetLastError());
   }
   ARGOT_CUDA_TRY(cudaEventRecord(b->ev[1 + parts], side));

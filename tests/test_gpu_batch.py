@@ -119,3 +119,19 @@ def test_batch_parts_of_few_and_many_blocks(cuda_ok, blocks_per_item):
         assert all(torch.equal(r, w) for r, w in zip(b.rates, want))
     b.check_device_error()
     b.close()
+
+
+def test_batch_of_many_tiny_problems_in_long_tiles(cuda_ok):
+    """Tiles much longer than the problems: a part's blocks are handed out one
+    by one without a unit per block that a tile could have had."""
+    import torch
+    from argot_b200 import workload as W
+    from argot_b200.batch import Batch
+    b = Batch([W.tiny(4 + i % 5, 1 + i % 3, seed=i) for i in range(40)])
+    want = [pb.run().clone() for pb in b.problems]
+    b.configure(mode=1, parts=3, blocks_per_item=4096)
+    _clear(b)
+    b.run()
+    assert all(torch.equal(r, w) for r, w in zip(b.rates, want))
+    b.check_device_error()
+    b.close()
