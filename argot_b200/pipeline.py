@@ -217,10 +217,10 @@ class Problem:
 
         overlap = P > 1 (one group whose buffers hold all rays): the group
         is cut into P parts along its blocks; the march of part p+1 runs on
-        one stream while the rates of part p run on another, so the
-        latency-bound march and the MUFU-bound rate kernel share the GPU at
-        each hand-over.  Same arithmetic: the result equals overlap = 0 bit
-        for bit.  The caller's current stream is ordered after all of it."""
+        one stream while the rates of part p run on another, so the march
+        (L1 data pipe, issue) and the rates (FMA pipe) share the SMs.  Same
+        arithmetic: the result equals overlap = 0 bit for bit.  The caller's
+        current stream is ordered after all of it."""
         if rates6 is None:
             rates6 = torch.zeros(6 * self.ncell, dtype=torch.float32, device=self.device)
         rays, tau = buffers if buffers is not None else self.alloc_group_buffers()

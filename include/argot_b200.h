@@ -341,8 +341,8 @@ ARGOT_B200_API int argot_b200_photoion_rays(const argot_b200_grid *g, const void
  * generation (emit = 1), then march and rates, the group's blocks [b0, b1)
  * cut into `parts` ranges of about equal ray counts (blk_offsets_host, the
  * host copy of blk_offsets_dev); the march of part p+1 runs on one internal
- * stream while the rates of part p run on another, so the latency-bound
- * march and the SFU-bound rates share the GPU.  rays_dev / tau_dev hold the
+ * stream while the rates of part p run on another, so the march (L1 data
+ * pipe) and the rates (FMA pipe) share the GPU.  rays_dev / tau_dev hold the
  * group's rays from `base` (tau: part p's three column planes start at
  * 3 x its first ray).  The result equals the separate calls bit for bit;
  * `stream` is ordered after all of it (and may be under graph capture). */
